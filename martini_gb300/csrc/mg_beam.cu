@@ -7,12 +7,23 @@
 // direct form here gives the same sums in FP32:
 //   out[i][j] = scale * sum_{a,b} in[i + hx - a][j + hy - b] * K[a][b],
 // hx = (kx - 1) / 2, hy = (ky - 1) / 2, zero outside the padded cube, for the
-// unpadded pixels only.  A block computes 8 x 16 output pixels of 32
-// channels (the cube's channel axis is the fastest, so a warp's lanes read 32
-// consecutive floats): the input halo tile and the beam image are staged in
-// shared memory; each thread accumulates one output row of 16 pixels for its
-// channel.  Beams whose halo tile does not fit read the cube through the
-// cache instead.
+// unpadded pixels only.
+//
+// k_beam_conv: a block computes 16 x 16 output pixels of 32 channels (the
+// cube's channel axis is the fastest, so a lane is a channel); each of its 8
+// warps holds two output rows, 32 sums a lane.  The work is bound by FP32 FMAs
+// (729 a voxel for a 27 px beam), so an input value must be read from shared
+// memory once for many of them: a lane loads a window of 16 + T - 1 pixels and
+// applies T = 8 taps of two kernel rows to it, 128 paired FMAs for 23 loads (one
+// load per FMA before: 9.70 ms on 512 x 512 x 256 with a 27 px beam; now
+// 2.29 ms, 1.23 ms of it at the FP32 FMA rate).  Input rows stream through a ring in shared memory (cp.async,
+// BR_AHEAD rows ahead): at step s warp w takes input row 2 w + s, so that every
+// warp works on kernel rows kx - 1 - s and kx - s and only 15 rows are live.
+// That leaves room for two blocks on an SM, and the ring's size depends on ky
+// mostly, so beams up to 71 px take this path (27 px before).  Each kernel row
+// is summed from zero and added to the voxel's total, which keeps the FP32
+// error below that of one running sum over all taps.
+// k_beam_conv_direct: wider beams, through the cache.
 #include <string>
 
 #include "mg_internal.cuh"
@@ -23,63 +34,199 @@ void set_last_error(const std::string& msg);  // mg_api.cu
 
 namespace {
 
-constexpr int BT_I = 8;   // output rows per block (one per warp)
-constexpr int BT_J = 16;  // output columns per thread
-constexpr int BC = 32;    // channels per block (one per lane)
-constexpr size_t kBeamSmemMax = 200 * 1024;
+constexpr int BT_I = 16;    // output rows per block, two per warp
+constexpr int BT_J = 16;    // output columns per thread
+constexpr int BC = 32;      // channels per block (one per lane)
+constexpr int BR_LIVE = BT_I - 1;  // input rows in use at a step
+constexpr int BR_AHEAD = 2;        // input rows in flight
+constexpr int BR_RING = BR_LIVE + BR_AHEAD;
+constexpr int BEAM_THREADS = BT_I / 2 * 32;
+constexpr size_t kBeamSmemMax = 226 * 1024;
 
+__host__ __device__ inline int beam_kstride(int ky) { return (ky + 3) & ~3; }
 size_t beam_smem(int kx, int ky) {
-  return sizeof(float) * ((size_t)(BT_I + kx - 1) * (BT_J + ky - 1) * BC + (size_t)kx * ky);
+  return sizeof(float) *
+         ((size_t)BR_RING * (BT_J + ky - 1) * BC + 2 * (size_t)(kx + 1) * beam_kstride(ky));
 }
 
-__global__ void __launch_bounds__(BT_I * 32) k_beam_conv(const float* __restrict__ in, int nx,
-                                                         int ny, int nc, int px, int py,
-                                                         const float* __restrict__ kern, int kx,
-                                                         int ky, float scale,
-                                                         float* __restrict__ out) {
-  extern __shared__ float sm[];
-  const int hi = BT_I + kx - 1, hj = BT_J + ky - 1;
-  float* s_in = sm;
-  float* s_k = sm + (size_t)hi * hj * BC;
-  const int hx = (kx - 1) / 2, hy = (ky - 1) / 2;
-  const int i0 = px + blockIdx.y * BT_I, j0 = py + blockIdx.x * BT_J, c0 = blockIdx.z * BC;
-  const int rb = i0 - hx, cb = j0 - hy;
-  const int tid = threadIdx.x;
-  const int total = hi * hj * BC;
-  for (int e = tid; e < total; e += blockDim.x) {
-    const int c = e % BC;
-    const int pc = e / BC;
-    const int r = pc / hj, q = pc - (pc / hj) * hj;
-    const int gi = rb + r, gj = cb + q, gc = c0 + c;
-    float v = 0.f;
-    if (gi >= 0 && gi < nx && gj >= 0 && gj < ny && gc < nc)
-      v = __ldg(in + ((long long)gi * ny + gj) * nc + gc);
-    s_in[e] = v;
+// Two FP32 values in a register pair: one instruction does both FMAs (each
+// rounds as the scalar FMA does).
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 f2_make(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_split(f2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// Taps b0 .. b0 + T - 1 of a step's kernel-row pair kp[b] = (row of output row
+// 0, row of output row 1) on the input row at `in` (this lane's channel):
+// acc[u] += in[u + ky - 1 - b] kp[b].
+template <int T>
+__device__ __forceinline__ void beam_taps(const float* in, const f2* kp, int b0, int ky,
+                                          f2 (&acc)[BT_J]) {
+  const float* col = in + (size_t)(ky - b0 - T) * BC;
+  float v[BT_J + T - 1];
+#pragma unroll
+  for (int q = 0; q < BT_J + T - 1; ++q) v[q] = col[q * BC];
+  f2 k[T];
+  if constexpr (T % 2 == 0) {
+#pragma unroll
+    for (int e = 0; e < T; e += 2) {
+      const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(kp + b0 + e);
+      k[e] = t.x;
+      k[e + 1] = t.y;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < T; ++e) k[e] = kp[b0 + e];
   }
-  for (int t = tid; t < kx * ky; t += blockDim.x) s_k[t] = kern[t];
-  __syncthreads();
-  const int lane = tid & 31, w = tid >> 5;
-  const int i = i0 + w;
-  if (i >= nx - px) return;
+#pragma unroll
+  for (int q = 0; q < BT_J + T - 1; ++q) {
+    const f2 x = f2_make(v[q], v[q]);
+#pragma unroll
+    for (int e = 0; e < T; ++e) {
+      const int u = q - (T - 1) + e;
+      if (u >= 0 && u < BT_J) acc[u] = f2_fma(x, k[e], acc[u]);
+    }
+  }
+}
+
+// One input row: the row sums of both output rows, added to their totals.
+__device__ __forceinline__ void beam_row(const float* in, const f2* kp, int ky, f2 (&tot)[BT_J]) {
+  f2 acc[BT_J];
+#pragma unroll
+  for (int u = 0; u < BT_J; ++u) acc[u] = 0ull;
+  int b = 0;
+#pragma unroll 1
+  for (; b + 8 <= ky; b += 8) beam_taps<8>(in, kp, b, ky, acc);
+  if (ky - b >= 4) {
+    beam_taps<4>(in, kp, b, ky, acc);
+    b += 4;
+  }
+#pragma unroll 1
+  for (; b < ky; ++b) beam_taps<1>(in, kp, b, ky, acc);
+#pragma unroll
+  for (int u = 0; u < BT_J; ++u) tot[u] = f2_add(tot[u], acc[u]);
+}
+
+// The first and last steps, where one of the two output rows (H) has no
+// kernel row: the other's sums only (no product of an input with a zero that
+// is not a tap).
+template <int H>
+__device__ __forceinline__ void beam_row1(const float* in, const f2* kp, int ky, f2 (&tot)[BT_J]) {
   float acc[BT_J];
 #pragma unroll
   for (int u = 0; u < BT_J; ++u) acc[u] = 0.f;
-  for (int a = 0; a < kx; ++a) {
-    const float* row = s_in + (size_t)(w + kx - 1 - a) * hj * BC + lane;
-    for (int b = 0; b < ky; ++b) {
-      const float kv = s_k[a * ky + b];
-      const float* col = row + (size_t)(ky - 1 - b) * BC;
+#pragma unroll 1
+  for (int b = 0; b < ky; ++b) {
+    const float2 k = f2_split(kp[b]);
 #pragma unroll
-      for (int u = 0; u < BT_J; ++u) acc[u] = fmaf(col[u * BC], kv, acc[u]);
-    }
+    for (int u = 0; u < BT_J; ++u)
+      acc[u] = fmaf(in[(size_t)(u + ky - 1 - b) * BC], H ? k.x : k.y, acc[u]);
   }
+#pragma unroll
+  for (int u = 0; u < BT_J; ++u) {
+    const float2 t = f2_split(tot[u]);
+    tot[u] = H ? f2_make(t.x + acc[u], t.y) : f2_make(t.x, t.y + acc[u]);
+  }
+}
+
+// VEC: 16-byte copies (nc a multiple of 4 and the cube 16-byte aligned).
+template <bool VEC>
+__global__ void __launch_bounds__(BEAM_THREADS, 2)
+k_beam_conv(const float* __restrict__ in, int nx, int ny, int nc, int px, int py,
+            const float* __restrict__ kern, int kx, int ky, float scale,
+            float* __restrict__ out) {
+  extern __shared__ __align__(16) float sm[];
+  const int hj = BT_J + ky - 1, ks = beam_kstride(ky);
+  float* const ring = sm;
+  f2* const s_k = reinterpret_cast<f2*>(sm + (size_t)BR_RING * hj * BC);
+  const int i0 = px + blockIdx.y * BT_I, j0 = py + blockIdx.x * BT_J, c0 = blockIdx.z * BC;
+  const int rb = i0 - (kx - 1) / 2, cb = j0 - (ky - 1) / 2;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int nrows = BT_I + kx - 1;
+  auto load_row = [&](int r) {  // input row r of the block into its ring slot
+    if (r < nrows) {
+      const int gi = rb + r;
+      const bool row_in = gi >= 0 && gi < nx;
+      const float* const src = in + (long long)(row_in ? gi : 0) * ny * nc;
+      float* const dst = ring + (size_t)(r % BR_RING) * hj * BC;
+      constexpr int V = VEC ? 4 : 1;
+      for (int e = tid; e < hj * (BC / V); e += BEAM_THREADS) {
+        const int q = e / (BC / V), c = (e - q * (BC / V)) * V;
+        const int gj = cb + q;
+        const bool ok = row_in && gj >= 0 && gj < ny && c0 + c < nc;
+        const float* g = ok ? src + (long long)gj * nc + c0 + c : in;
+        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + q * BC + c);
+        if (VEC)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(g),
+                       "r"(ok ? 16 : 0)
+                       : "memory");
+        else
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(g),
+                       "r"(ok ? 4 : 0)
+                       : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int r = 0; r < BR_LIVE - 1; ++r) load_row(r);
+  for (int r = 0; r < BR_AHEAD; ++r) load_row(BR_LIVE - 1 + r);
+  // s_k[s][b]: the kernel rows of step s, kx - 1 - s and kx - s, as pairs
+  for (int t = tid; t < (kx + 1) * ks; t += BEAM_THREADS) {
+    const int st = t / ks, b = t - st * ks;
+    const int a0 = kx - 1 - st;
+    s_k[t] = f2_make(b < ky && a0 >= 0 ? kern[a0 * ky + b] : 0.f,
+                     b < ky && a0 + 1 < kx ? kern[(a0 + 1) * ky + b] : 0.f);
+  }
+  f2 tot[BT_J];
+#pragma unroll
+  for (int u = 0; u < BT_J; ++u) tot[u] = 0ull;
+  for (int s = 0; s <= kx; ++s) {
+    // row s + BR_LIVE - 1 has arrived; every warp is done with row s - 1,
+    // whose slot the next row takes
+    asm volatile("cp.async.wait_group %0;" ::"n"(BR_AHEAD - 1) : "memory");
+    __syncthreads();
+    load_row(s + BR_LIVE - 1 + BR_AHEAD);
+    const float* row = ring + (size_t)((2 * w + s) % BR_RING) * hj * BC + lane;
+    const f2* kp = s_k + (size_t)s * ks;
+    if (s == 0)
+      beam_row1<1>(row, kp, ky, tot);
+    else if (s == kx)
+      beam_row1<0>(row, kp, ky, tot);
+    else
+      beam_row(row, kp, ky, tot);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   const int c = c0 + lane;
   if (c >= nc) return;
   const int nyo = ny - 2 * py;
 #pragma unroll
-  for (int u = 0; u < BT_J; ++u) {
-    const int j = j0 + u;
-    if (j < ny - py) out[((long long)(i - px) * nyo + (j - py)) * nc + c] = acc[u] * scale;
+  for (int h = 0; h < 2; ++h) {
+    const int i = i0 + 2 * w + h;
+    if (i >= nx - px) continue;
+#pragma unroll
+    for (int u = 0; u < BT_J; ++u) {
+      const int j = j0 + u;
+      const float2 t = f2_split(tot[u]);
+      if (j < ny - py)
+        out[((long long)(i - px) * nyo + (j - py)) * nc + c] = (h ? t.y : t.x) * scale;
+    }
   }
 }
 
@@ -123,16 +270,18 @@ extern "C" int mg_convolve_beam(const float* cube, int32_t nx, int32_t ny, int32
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t smem = beam_smem(kx, ky);
   if (smem <= kBeamSmemMax) {
+    const bool vec = (nc & 3) == 0 && (reinterpret_cast<uintptr_t>(cube) & 15) == 0;
+    const auto kernel_fn = vec ? k_beam_conv<true> : k_beam_conv<false>;
     if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(k_beam_conv, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(kernel_fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kBeamSmemMax) != cudaSuccess) {
       mg::set_last_error("mg_convolve_beam: shared memory attribute");
       return MG_ERR_CUDA;
     }
     const dim3 grid((unsigned)((ny - 2 * pady + BT_J - 1) / BT_J),
                     (unsigned)((nx - 2 * padx + BT_I - 1) / BT_I), (unsigned)((nc + BC - 1) / BC));
-    k_beam_conv<<<grid, BT_I * 32, smem, s>>>(cube, nx, ny, nc, padx, pady, kernel, kx, ky, scale,
-                                              out);
+    kernel_fn<<<grid, BEAM_THREADS, smem, s>>>(cube, nx, ny, nc, padx, pady, kernel, kx, ky, scale,
+                                               out);
   } else {
     k_beam_conv_direct<<<4096, 256, 0, s>>>(cube, nx, ny, nc, padx, pady, kernel, kx, ky, scale,
                                             out);
