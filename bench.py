@@ -54,27 +54,43 @@ FORMS = {"fp32": 0, "bf16x3": 1, "f16x3": 2, "bf16x6": 3}
 TRAFFIC_BYTES = {("disc4m_1024", "bf16x6"): 5_896_006_400}
 
 
-def launches_per_step(form: str, gaussian: bool, nx: int, ny: int, nc: int, ngal: int = 1,
-                      ntiles: int | None = None) -> int:
+def launches_per_step(form: str, gaussian: bool, nx: int, ny: int, nc: int, n: int, pairs: int,
+                      ngal: int = 1, ntiles: int | None = None, nseg: int | None = None) -> int:
     """Kernels one mg_insert(_batched) launches: cube table (one per 16
-    cubes), tile init, edges, prep, pair scan (3), difference-array prefix,
-    tile scan (3), plan, emit, radix passes x (histogram, scan (3), scatter),
-    segments, item and partial scans (2 x 3), work-queue keys and their two
-    radix passes (2 x 5), partial check, [spectrum store: row lengths, scan
-    (3), rows], [cube clear for batches], [tensor-core parameters],
-    contraction, split-K reduction, flux (3)."""
+    cubes), tile init, edges, prep, pair scan, difference-array prefix, tile
+    scan, plan, the particle order (a distribution pass), the pair scan in that
+    order, emit, the segment passes, segments, item and partial scans,
+    work-queue keys and their pass, partial check, [spectrum store: row
+    lengths, scan, rows], [cube clear for batches], [tensor-core parameters],
+    contraction, split-K reduction, flux (3).  A scan is one launch up to 8192
+    entries, else three; a pass one launch up to two tiles of 8192 elements,
+    else a histogram, a scan and the scatter."""
     if ntiles is None:
         ntiles = ((nx + 7) // 8) * ((ny + 15) // 16)  # 8 x 16-pixel tiles
-    bits = max(ntiles - 1, 0).bit_length() + max(nc - 1, 0).bit_length()
-    passes = (bits + 7) // 8
-    n = (ngal + 15) // 16 + 1 + 1 + 1 + 3 + 1 + 3 + 1 + 1 + 5 * passes + 1 + 6 + 1 + 10 + 1
+    if nseg is None:
+        width = {"fp32": 64, "bf16x6": 128}.get(form, 256)
+        nseg = ntiles * max(1, -(-nc // width))
+
+    def scan(m):
+        return 1 if m <= 8192 else 3
+
+    def dist(m, bits):
+        t = -(-m // 8192)
+        return 1 if t <= 2 else 2 + scan(min(t, 1216) << max(bits, 1))
+
+    bits = max(nseg - 1, 0).bit_length()
+    passes = max(1, -(-bits // 9))
+    items = min(pairs, nseg + pairs // 2048 + 1)
+    k = (ngal + 15) // 16 + 1 + 1 + 1 + scan(n) + 1 + scan(ntiles) + 1
+    k += dist(n, 9) + scan(n) + 1 + passes * dist(pairs, -(-bits // passes)) + 1
+    k += 2 * scan(nseg) + 1 + dist(items, 9) + 1
     if form != "fp32" and gaussian:
-        n += 1 + 3 + 1
+        k += 1 + scan(n) + 1
     if form != "fp32":
-        n += 1
+        k += 1
     if ngal > 1:
-        n += 1
-    return n + 1 + 1 + 3
+        k += 1
+    return k + 1 + 1 + 3
 
 
 def parse():
@@ -524,7 +540,8 @@ def main():
         "e2e": {"value": 1.0 / t_e2e, "unit": "cubes/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h)},
         "gpu_launches": a.steps * sum(launches_per_step(
-            a.form, g["prob"].spectral_model == N.MG_SPECTRUM_GAUSSIAN, nx, ny, nc) for g in ins),
+            a.form, g["prob"].spectral_model == N.MG_SPECTRUM_GAUSSIAN, nx, ny, nc,
+            int(g["prob"].n), int(g["info"].n_pairs)) for g in ins),
         "step_ms": [round(t * 1e3, 3) for t in t_step],
         "clocks": clk,
     }
@@ -868,8 +885,11 @@ def run_population(a, rank, world, local, dev):
         "roofline": rl,
         "e2e": {"value": ng / t_e2e, "unit": "cubes/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h)},
-        "gpu_launches": a.steps * launches_per_step(a.form, True, 0, 0,
-                                                    max(w["nc"] for w in gals), ng, ntiles),
+        "gpu_launches": a.steps * launches_per_step(
+            a.form, True, 0, 0, max(w["nc"] for w in gals), sum(w["n"] for w in gals),
+            int(info.n_pairs), ng, ntiles,
+            sum(-(-w["nx"] // 8) * -(-w["ny"] // 16)
+                * -(-w["nc"] // {"fp32": 64, "bf16x6": 128}.get(a.form, 256)) for w in gals)),
         "step_ms": [round(t * 1e3, 3) for t in t_batch],
         "clocks": clk,
     }

@@ -82,9 +82,11 @@ Layout layout(const Geo& g, long long cap_pairs, long long cap_partial) {
   const size_t nn = (size_t)(g.n > 0 ? g.n : 1);
   const size_t ng1 = (size_t)g.ngal + 1;
   const size_t cp = (size_t)(cap_pairs > 0 ? cap_pairs : 1);
-  const long long rb = radix_blocks(cap_pairs > 0 ? cap_pairs : 1);
+  // (a pass of one chunk keeps its counts in shared memory)
+  const long long chunks = radix_chunks(cap_pairs > 0 ? cap_pairs : 1);
+  const long long rb = chunks > 1 ? chunks << RS_BITS : 0;
   long long scan_n = g.n;
-  if (256 * rb > scan_n) scan_n = 256 * rb;
+  if (rb > scan_n) scan_n = rb;
   if (g.nseg > scan_n) scan_n = g.nseg;
   if (g.ntiles > scan_n) scan_n = g.ntiles;
   L.hdr = take(sizeof(WsHeader));
@@ -110,8 +112,8 @@ Layout layout(const Geo& g, long long cap_pairs, long long cap_partial) {
   L.list = take(sizeof(int) * cp);
   L.keys_tmp = take(sizeof(unsigned) * cp);
   L.list_tmp = take(sizeof(int) * cp);
-  L.rs_hist = take(sizeof(int) * 256 * (size_t)rb);
-  L.rs_off = take(sizeof(long long) * 256 * (size_t)rb);
+  L.rs_hist = take(sizeof(int) * (size_t)rb);
+  L.rs_off = take(sizeof(long long) * (size_t)rb);
   L.scan_sums = take(sizeof(long long) * (size_t)(scan_blocks(scan_n) + 1));
   L.seg_lo = take(sizeof(long long) * (size_t)g.nseg);
   L.seg_hi = take(sizeof(long long) * (size_t)g.nseg);

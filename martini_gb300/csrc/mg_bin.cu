@@ -374,53 +374,45 @@ __device__ __forceinline__ int div_exact(int a, int b, float rb) {
   return q;
 }
 
-// Pairs in particle order: key = global segment << cbits | class << (cbits -
-// 2) | clo, class 0 for the table kernels, 1 for the Dirac kernel, 2 for the
-// Gaussian and cubic-spline kernels (each class's particles then form
-// stages of their own in each segment, which the tensor-core producers take
-// on the class's own path) (one pair per
-// tile and channel block the particle's line meets), value = particle.  A
-// warp takes 32 particles, whose pairs are one contiguous range of the
-// output (pair_off is the exclusive scan of the counts); each lane writes
-// every 32nd pair of the range, finding its particle by a search over the
-// lanes' first pairs, so every store of the warp is contiguous.  Pair e of
-// a particle enumerates its tiles row-major over (tx, ty), then its channel
-// blocks, at position pair_off[P] + e.
-__global__ void k_emit(Geo g, Ws w, unsigned* __restrict__ keys, int* __restrict__ vals) {
+// Pairs in the order of `order` (particles by kernel class and first channel):
+// key = global segment, value = particle, one pair per tile and channel block
+// the particle's line meets.  A warp takes 32 particles, whose pairs are one
+// contiguous range of the output (pair_off is the exclusive scan of the counts
+// in this order); each lane writes every 32nd pair of the range, finding its
+// particle by a search over the lanes' first pairs, so every store of the warp
+// is contiguous.  Pair e of a particle enumerates its tiles row-major over
+// (tx, ty), then its channel blocks.
+__global__ void k_emit(Geo g, Ws w, const int* __restrict__ order, unsigned* __restrict__ keys,
+                       int* __restrict__ vals) {
   if (w.hdr->status & (ST_PAIRS | ST_EDGES)) return;
   const int lane = threadIdx.x & 31;
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+  const long long nv = w.hdr->n_valid;
   for (long long base = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * 32;
-       base < g.n; base += nwarps * 32) {
-    const long long P = base + lane;
+       base < nv; base += nwarps * 32) {
+    const long long K = base + lane;
     // this lane's particle: first pair, pair count and the parameters of its
     // tile / block ranges
     long long o = 0x7fffffffffffffffll;  // lanes past the end never match
-    int np = 0, tx0 = 0, ty0 = 0, nty_span = 1, cb0 = 0, nb = 1, clo = 0, seg0 = 0, nty = 1,
-        ncb = 1;
-    unsigned cls = 0u;
-    if (P < g.n) {
-      o = w.pair_off[P];
+    int P = 0, np = 0, tx0 = 0, ty0 = 0, nty_span = 1, cb0 = 0, nb = 1, seg0 = 0, nty = 1, ncb = 1;
+    if (K < nv) {
+      P = order[K];
+      o = w.pair_off[K];
       np = w.npairs[P];
-      if (np > 0) {
+      {
         const PRec rec = w.rec[P];
-        const Gal& G = w.gal[find_gal(w.gp0, g.ngal, P)];
+        const Gal& G = w.gal[find_gal(w.gp0, g.ngal, (long long)P)];
         tx0 = rec.ilo / TILE_I;
         ty0 = rec.jlo / TILE_J;
         nty_span = rec.jhi / TILE_J - ty0 + 1;
         cb0 = G.ncb > 1 ? rec.clo / G.width : 0;
         nb = G.ncb > 1 ? rec.chi / G.width - cb0 + 1 : 1;
-        clo = rec.clo;
-        const int kt = g.ks[rec.kslot].type;
-        cls = (kt == MG_KERNEL_GAUSSIAN || kt == MG_KERNEL_CUBIC_SPLINE) ? 2u
-              : kt == MG_KERNEL_DIRAC                                     ? 1u
-                                                                          : 0u;
         seg0 = G.seg0;
         nty = G.nty;
         ncb = G.ncb;
       }
     }
-    const int last = (int)min(31ll, g.n - 1 - base);
+    const int last = (int)min(31ll, nv - 1 - base);
     const long long start = __shfl_sync(0xffffffffu, o, 0);
     const long long end = __shfl_sync(0xffffffffu, o + np, last);
     for (long long f0 = start; f0 < end; f0 += 32) {  // warp-uniform
@@ -439,8 +431,7 @@ __global__ void k_emit(Geo g, Ws w, unsigned* __restrict__ keys, int* __restrict
       const int sspan = __shfl_sync(0xffffffffu, nty_span, src);
       const int scb0 = __shfl_sync(0xffffffffu, cb0, src);
       const int snb = __shfl_sync(0xffffffffu, nb, src);
-      const int sclo = __shfl_sync(0xffffffffu, clo, src);
-      const unsigned scls = __shfl_sync(0xffffffffu, cls, src);
+      const int sP = __shfl_sync(0xffffffffu, P, src);
       const int sseg0 = __shfl_sync(0xffffffffu, seg0, src);
       const int snty = __shfl_sync(0xffffffffu, nty, src);
       const int sncb = __shfl_sync(0xffffffffu, ncb, src);
@@ -453,45 +444,52 @@ __global__ void k_emit(Geo g, Ws w, unsigned* __restrict__ keys, int* __restrict
         }
         const int a = div_exact(t, sspan, __frcp_rn((float)sspan));
         const int tx = stx0 + a, ty = sty0 + (t - a * sspan);
-        const unsigned sg = (unsigned)(sseg0 + (tx * snty + ty) * sncb + cb);
-        keys[f] = (sg << g.cbits) | (scls << (g.cbits - 2)) | (unsigned)sclo;
-        vals[f] = (int)(base + src);
+        keys[f] = (unsigned)(sseg0 + (tx * snty + ty) * sncb + cb);
+        vals[f] = sP;
       }
     }
   }
 }
 
-// First index in [lo, hi) of sorted keys with key >= k.
+// First index in [lo, hi) of sorted keys with key >= k, by a warp: 32 probes a
+// round (a thread's bisection is 15 to 27 dependent reads, which took 15 us
+// even for a list of 30,000 pairs).
 __device__ __forceinline__ long long lower_bound_keys(const unsigned* keys, long long lo,
-                                                      long long hi, unsigned k) {
+                                                      long long hi, unsigned k, int lane) {
   while (lo < hi) {
-    long long m = (lo + hi) >> 1;
-    if (keys[m] < k) lo = m + 1; else hi = m;
+    const long long step = (hi - lo + 31) / 32;
+    const long long m = lo + lane * step;  // probes in ascending order
+    const bool less = m < hi && keys[m] < k;
+    const int n = __popc(__ballot_sync(0xffffffffu, less));  // the first n probes are less
+    if (n == 0) return lo;
+    const long long last = lo + (long long)(n - 1) * step;  // the last one that is
+    hi = min(hi, last + step);
+    lo = last + 1;
   }
   return lo;
 }
 
-// One thread per segment (tile, channel block): its range of the sorted
-// list (keys segment << cbits | clo, so the segment's particles are exactly
-// the keys in [segment << cbits, (segment + 1) << cbits)), its K chunks and
-// its split-K partial items.
+// One warp per segment (tile, channel block): its range of the sorted list,
+// its K chunks and its split-K partial items.
 __global__ void k_segments(Geo g, Ws w) {
   const bool bad = (w.hdr->status & (ST_PAIRS | ST_EDGES)) != 0;
   const int kch = w.hdr->kch;
   const long long n = w.hdr->n_pairs;
-  for (int sg = blockIdx.x * blockDim.x + threadIdx.x; sg < g.nseg; sg += gridDim.x * blockDim.x) {
-    long long lo = 0, hi = 0;
-    int items = 0, part = 0;
-    if (!bad && n > 0) {
-      lo = lower_bound_keys(w.keys, 0, n, (unsigned)sg << g.cbits);
-      hi = sg + 1 == g.nseg ? n
-                            : lower_bound_keys(w.keys, lo, n, (unsigned)(sg + 1) << g.cbits);
-      const long long cnt = hi - lo;
-      if (cnt > 0) {
-        items = (int)((cnt + kch - 1) / kch);
-        part = items > 1 ? items : 0;
-      }
+  const int lane = threadIdx.x & 31;
+  const int sg = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
+  if (sg >= g.nseg) return;
+  long long lo = 0, hi = 0;
+  int items = 0, part = 0;
+  if (!bad && n > 0) {
+    lo = lower_bound_keys(w.keys, 0, n, (unsigned)sg, lane);
+    hi = sg + 1 == g.nseg ? n : lower_bound_keys(w.keys, lo, n, (unsigned)sg + 1u, lane);
+    const long long cnt = hi - lo;
+    if (cnt > 0) {
+      items = (int)((cnt + kch - 1) / kch);
+      part = items > 1 ? items : 0;
     }
+  }
+  if (lane == 0) {
     w.seg_lo[sg] = lo;
     w.seg_hi[sg] = hi;
     w.seg_items[sg] = items;
@@ -503,13 +501,14 @@ __global__ void k_segments(Geo g, Ws w) {
 // (item k of a segment holds min(kch, cnt - k kch) particles).  Estimated
 // cost = particles x (2 TILE_PX + width): the kernel weights at the tile's
 // pixels and the spectra and products over the segment's channel block.
-// Key = 65535 - cost scaled to 16 bits, so that the stable ascending radix
-// sort puts the largest items first and keeps segment order among equal
-// ones: the persistent contraction then ends on the small items instead of
-// leaving one large item to a single SM at the end.
+// Key = top - cost scaled to RS_BITS bits, so that one stable distribution
+// pass puts the largest items first and keeps segment order among equal ones:
+// the persistent contraction then ends on the small items instead of leaving
+// one large item to a single SM at the end.
 __global__ void k_item_keys(Geo g, Ws w) {
   if (w.hdr->status & (ST_PAIRS | ST_EDGES)) return;
   const int kch = w.hdr->kch;
+  const double top = (double)((1 << RS_BITS) - 1);
   const double cmax = (double)kch * (2.0 * TILE_PX + (double)g.max_width);
   for (int sg = blockIdx.x * blockDim.x + threadIdx.x; sg < g.nseg; sg += gridDim.x * blockDim.x) {
     const int n_it = w.seg_items[sg];
@@ -520,11 +519,11 @@ __global__ void k_item_keys(Geo g, Ws w) {
     for (int k = 0; k < n_it && base + k < w.cap_items; ++k) {
       const long long left = cnt - (long long)k * kch;
       const double lc = (double)(left < kch ? left : kch);
-      double q = lc * (2.0 * TILE_PX + (double)width) / cmax * 65535.0 + 0.5;
-      if (q > 65535.0) q = 65535.0;
+      double q = lc * (2.0 * TILE_PX + (double)width) / cmax * top + 0.5;
+      if (q > top) q = top;
       // all keys equal: the stable sort keeps segment order
-      w.item_key[base + k] = g.cost_order ? 65535u - (unsigned)q : 0u;
-      w.item_order[base + k] = (int)(base + k);
+      w.item_key_tmp[base + k] = g.cost_order ? (unsigned)top - (unsigned)q : 0u;
+      w.item_order_tmp[base + k] = (int)(base + k);
       w.item_seg[base + k] = sg;
     }
   }
@@ -576,33 +575,54 @@ void launch_prep(const Geo& g, const Ws& w, int num_sms, cudaStream_t s, long lo
   k_plan_finish<<<grid_for(g.ntiles, num_sms), 256, 0, s>>>(g, w, num_sms);
 }
 
-int sort_bits(const Geo& g) {
-  int sbits = 0;
-  while ((1LL << sbits) < (long long)g.nseg) ++sbits;
-  return sbits + g.cbits;
+int seg_bits(const Geo& g) {
+  int b = 0;
+  while ((1LL << b) < (long long)g.nseg) ++b;
+  return b;
 }
 
-// Tile-major list sorted by (tile, clo), then the segments with their
-// work-item and partial offsets.  Pairs are emitted into the buffer from
-// which an even/odd number of radix passes ends in w.keys / w.list.
+int sort_bits(const Geo& g) { return seg_bits(g) + g.cbits; }
+
+// The list sorted by segment, then class and first channel, then the segments
+// with their work-item and partial offsets.  Pairs are emitted into the buffer
+// from which an even/odd number of passes ends in w.keys / w.list; the
+// particle order lies in the other buffer's keys until the first pass.
 void launch_sort_segments(const Geo& g, const Ws& w, long long cap_pairs, int num_sms,
                           cudaStream_t s) {
-  const int passes = (sort_bits(g) + 7) / 8;
-  unsigned* k0 = (passes & 1) ? w.keys_tmp : w.keys;
-  int* v0 = (passes & 1) ? w.list_tmp : w.list;
-  unsigned* k1 = (passes & 1) ? w.keys : w.keys_tmp;
-  int* v1 = (passes & 1) ? w.list : w.list_tmp;
-  if (g.n > 0) k_emit<<<grid_for(g.n, num_sms), 256, 0, s>>>(g, w, k0, v0);
-  launch_radix_sort(k0, v0, k1, v1, &w.hdr->n_pairs, cap_pairs, sort_bits(g), w.rs_hist,
-                    w.rs_off, w.scan_sums, num_sms, s);
-  k_segments<<<(unsigned)((g.nseg + 255) / 256), 256, 0, s>>>(g, w);
+  const int bits = seg_bits(g);
+  const bool odd = (radix_passes(bits) & 1) != 0;
+  unsigned* k0 = odd ? w.keys_tmp : w.keys;
+  int* v0 = odd ? w.list_tmp : w.list;
+  unsigned* k1 = odd ? w.keys : w.keys_tmp;
+  int* v1 = odd ? w.list : w.list_tmp;
+  if (g.n > 0) {
+    int* const order = reinterpret_cast<int*>(k1);  // n_valid <= pairs <= cap_pairs
+    // the particle pass's chunk counts: the pairs' scratch, or the flux sums'
+    // rows where a cube has more particles than pairs
+    const size_t per = (size_t)(sizeof(int) + sizeof(long long)) << RS_BITS;
+    int* hist = w.rs_hist;
+    long long* off = w.rs_off;
+    long long room = radix_chunks(cap_pairs > 0 ? cap_pairs : 1);
+    const long long froom = (long long)(sizeof(double) * (size_t)g.nfpart / per);
+    if (room < radix_chunks(g.n) && froom > room) {
+      room = froom;
+      off = reinterpret_cast<long long*>(w.flux_part);
+      hist = reinterpret_cast<int*>(off + (room << RS_BITS));
+    }
+    launch_order_particles(g, w, order, room, hist, off, s);
+    launch_scan_gather(w.npairs, order, &w.hdr->n_valid, g.n, w.pair_off, w.scan_sums, s);
+    k_emit<<<grid_for(g.n, num_sms), 256, 0, s>>>(g, w, order, k0, v0);
+  }
+  launch_radix_sort(k0, v0, k1, v1, &w.hdr->n_pairs, cap_pairs, bits, w.rs_hist, w.rs_off,
+                    w.scan_sums, s);
+  k_segments<<<(unsigned)((g.nseg + 7) / 8), 256, 0, s>>>(g, w);
   launch_scan(w.seg_items, g.nseg, w.item_off, w.scan_sums, &w.hdr->n_items, s);
   launch_scan(w.seg_part, g.nseg, w.part_off, w.scan_sums, &w.hdr->n_partial_items, s);
-  // the work queue: items by estimated cost, largest first (16-bit keys: two
-  // radix passes, the result back in item_key / item_order)
+  // the work queue: items by estimated cost, largest first (one pass, into
+  // item_key / item_order)
   k_item_keys<<<(unsigned)((g.nseg + 255) / 256), 256, 0, s>>>(g, w);
-  launch_radix_sort(w.item_key, w.item_order, w.item_key_tmp, w.item_order_tmp, &w.hdr->n_items,
-                    w.cap_items, 16, w.rs_hist, w.rs_off, w.scan_sums, num_sms, s);
+  launch_radix_sort(w.item_key_tmp, w.item_order_tmp, w.item_key, w.item_order, &w.hdr->n_items,
+                    w.cap_items, RS_BITS, w.rs_hist, w.rs_off, w.scan_sums, s);
   k_check_partials<<<1, 1, 0, s>>>(w);
 }
 

@@ -143,8 +143,7 @@ struct Geo {
   int nseg;           // segments of all cubes
   int max_width;      // widest channel block (partial slots hold TILE_PX x max_width)
   int max_nc;
-  int cbits;          // key bits below the segment: two kernel-class bits, then the
-                      // channel bits of the widest band
+  int cbits;          // class and channel bits of the order within a segment
   int nrows;          // flux rows of all cubes
   int max_diff;       // largest difference array of one cube
   long long n;        // particles of all cubes
@@ -194,7 +193,7 @@ struct WsHeader {
   long long n_spec;              // values in the spectrum store (spectrum stage)
   int spec_ready;                // 1 once the store holds this binning's spectra
   int kch;                       // particles per work item (item_particles)
-  long long pad1[1];
+  long long n_valid;             // particles with pairs (particle list stage)
 };
 
 // Pointers into the workspace (host computes, passes by value).  Arrays run
@@ -221,12 +220,12 @@ struct Ws {
   float* ehi;            // [nedge] edges, double-float high part
   float* elo;            // [nedge] low part
   float* inv_w;          // [nedge] 1 / |channel width| (channel c of a cube at edge0 + c)
-  unsigned* keys;        // [cap_pairs] sorted keys: segment << cbits | class | clo
+  unsigned* keys;        // [cap_pairs] sorted keys: segment
   int* list;             // [cap_pairs] particle ids in sorted order
   unsigned* keys_tmp;    // [cap_pairs] radix-sort second buffer
   int* list_tmp;         // [cap_pairs]
-  int* rs_hist;          // [256 * radix_blocks(cap_pairs)]
-  long long* rs_off;     // [256 * radix_blocks(cap_pairs)]
+  int* rs_hist;          // [2^RS_BITS * radix_chunks(cap_pairs)]
+  long long* rs_off;     // [2^RS_BITS * radix_chunks(cap_pairs)]
   long long* scan_sums;  // [scan scratch]
   long long* seg_lo;     // [nseg] list range of each segment
   long long* seg_hi;     // [nseg]
@@ -265,13 +264,20 @@ void launch_prep(const Geo& g, const Ws& w, int num_sms, cudaStream_t s, long lo
 void launch_sort_segments(const Geo& g, const Ws& w, long long cap_pairs, int num_sms,
                           cudaStream_t s);
 int sort_bits(const Geo& g);
+int seg_bits(const Geo& g);
 void launch_scan(const int* in, long long n, long long* out, long long* sums, long long* total,
                  cudaStream_t s);
+void launch_scan_gather(const int* in, const int* idx, const long long* m, long long n,
+                        long long* out, long long* sums, cudaStream_t s);
 long long scan_blocks(long long n);
-long long radix_blocks(long long n);
-bool launch_radix_sort(unsigned* keys, int* vals, unsigned* kt, int* vt, const long long* np,
+constexpr int RS_BITS = 9;  // widest digit of a distribution pass
+long long radix_chunks(long long n);
+int radix_passes(int bits);
+void launch_radix_sort(unsigned* keys, int* vals, unsigned* kt, int* vt, const long long* np,
                        long long cap, int bits, int* hist, long long* off, long long* sums,
-                       int num_sms, cudaStream_t s);
+                       cudaStream_t s);
+void launch_order_particles(const Geo& g, const Ws& w, int* out, long long max_chunks, int* hist,
+                            long long* off, cudaStream_t s);
 int launch_contract_fp32(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
 int launch_contract_bf16x3(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
 void launch_reduce_partials(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
