@@ -68,7 +68,7 @@ def launches_per_step(form: str, gaussian: bool, nx: int, ny: int, nc: int, n: i
     if ntiles is None:
         ntiles = ((nx + 7) // 8) * ((ny + 15) // 16)  # 8 x 16-pixel tiles
     if nseg is None:
-        width = {"fp32": 64, "bf16x6": 128}.get(form, 256)
+        width = 64 if form == "fp32" else 256
         nseg = ntiles * max(1, -(-nc // width))
 
     def scan(m):
@@ -889,7 +889,7 @@ def run_population(a, rank, world, local, dev):
             a.form, True, 0, 0, max(w["nc"] for w in gals), sum(w["n"] for w in gals),
             int(info.n_pairs), ng, ntiles,
             sum(-(-w["nx"] // 8) * -(-w["ny"] // 16)
-                * -(-w["nc"] // {"fp32": 64, "bf16x6": 128}.get(a.form, 256)) for w in gals)),
+                * -(-w["nc"] // (64 if a.form == "fp32" else 256)) for w in gals)),
         "step_ms": [round(t * 1e3, 3) for t in t_batch],
         "clocks": clk,
     }

@@ -37,13 +37,15 @@ bool known_form(int form) {
 }
 
 // Segment shape of a contraction form: channel blocks per tile and their
-// width.  Tensor-core forms: the band (rounded to 16) in one block up to the
-// form's block width, else blocks of that width: 256 for the pairs (a block
-// and its master accumulator fill the 512 TMEM columns), 128 for bf16x6
-// (two working accumulators and the master: its 64-particle stages).
-void seg_shape(int form, int nc, int* ncb, int* width) {
+// width.  Tensor-core forms: the band (rounded to 16) in one block up to 256
+// channels, else blocks of 256 (a block's master accumulator takes half of
+// the 512 TMEM columns).  `small_partials` (the built-in scratch of
+// mg_insert_noalloc) keeps the three-piece form at blocks of 128, whose
+// split-K partial tiles take half the room: a problem that fits the fixed
+// array with them may not fit with 256.
+void seg_shape(int form, int nc, bool small_partials, int* ncb, int* width) {
   if (form == MG_FORM_BF16X3 || form == MG_FORM_F16X3 || form == MG_FORM_BF16X6) {
-    const int bw = form == MG_FORM_BF16X6 ? 128 : 256;
+    const int bw = small_partials && form == MG_FORM_BF16X6 ? 128 : 256;
     if (nc <= bw) {
       *ncb = 1;
       *width = (nc + 15) / 16 * 16;
@@ -236,7 +238,8 @@ struct Batch {
 // contraction form and accumulate flag) and lay its cubes out in the
 // batch-wide index spaces.  `shape_only` (workspace sizing) checks just
 // what the layout depends on: sizes, pads and form.
-int make_batch(const mg_problem* probs, int nprob, Batch* b, bool shape_only = false) {
+int make_batch(const mg_problem* probs, int nprob, Batch* b, bool shape_only = false,
+               bool small_partials = false) {
   if (!probs || nprob < 1) return fail(MG_ERR_INVALID_ARGUMENT, "empty batch");
   if (nprob > 65535) return fail(MG_ERR_INVALID_ARGUMENT, "at most 65535 cubes in a batch");
   for (int k = 0; k < nprob; ++k) {
@@ -306,7 +309,7 @@ int make_batch(const mg_problem* probs, int nprob, Batch* b, bool shape_only = f
     G.ntx = (p.nx + TILE_I - 1) / TILE_I;
     G.nty = (p.ny + TILE_J - 1) / TILE_J;
     const long long nt = (long long)G.ntx * G.nty;
-    seg_shape(p.form, p.nc, &G.ncb, &G.width);
+    seg_shape(p.form, p.nc, small_partials, &G.ncb, &G.width);
     G.p0 = n;
     G.n = p.n;
     G.tile0 = (int)ntiles;
@@ -468,9 +471,9 @@ std::string class_key(const Batch& b, long long max_pairs) {
 // list to the binning stage); all asynchronous on stream s.
 int run(const mg_problem* probs, int nprob, void* ws, size_t bytes, cudaStream_t s,
         long long cap_pairs, long long cap_partial, int stages, bool scatter, Ws* wout,
-        Batch* bout, const mg_tuning* shape) {
+        Batch* bout, const mg_tuning* shape, bool small_partials = false) {
   Batch& b = *bout;
-  int rc = make_batch(probs, nprob, &b);
+  int rc = make_batch(probs, nprob, &b, false, small_partials);
   if (rc) return rc;
   apply_shape(shape, scatter, &b.g);
   const Geo& g = b.g;
@@ -518,6 +521,28 @@ int run(const mg_problem* probs, int nprob, void* ws, size_t bytes, cudaStream_t
 }
 
 }  // namespace
+
+namespace mg {
+
+// mg_workspace_size and mg_insert with small split-K partial tiles (seg_shape)
+int workspace_size_small(const mg_problem* p, long long max_pairs, long long max_partial,
+                             size_t* bytes) {
+  Batch b;
+  const int rc = make_batch(p, 1, &b, true, true);
+  if (!rc) *bytes = layout(b.g, max_pairs, max_partial).total;
+  return rc;
+}
+
+int insert_small(const mg_problem* p, void* ws, size_t bytes, long long max_pairs,
+                     long long max_partial, cudaStream_t s) {
+  Ws w;
+  Batch b;
+  mg_tuning shape;
+  mg_tuning_lookup(p, 1, max_pairs, &shape);
+  return run(p, 1, ws, bytes, s, max_pairs, max_partial, MG_STAGE_ALL, true, &w, &b, &shape, true);
+}
+
+}  // namespace mg
 
 extern "C" {
 

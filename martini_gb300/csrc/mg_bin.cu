@@ -73,11 +73,11 @@ void launch_set_gals(const Gal* gals, const Geo& g, const Ws& w, cudaStream_t s)
 // pixel within the kernel's support radius, so the tiles in the corners of a
 // wide box, where every weight is exactly zero, make no pairs: 17 % fewer
 // of them on 1M particles in 512^2 x 256 (20.8M to 17.3M, contraction 6.5 to
-// 5.7 ms), 20 % on 500k wide ones in 1024^2 x 256 (30.4 to 25.8 ms).  `reach2` is the squared radius in
-// px with a margin far above the rounding of the FP32 weights (2e-5 relative
-// and 2e-4 px); a kernel without a radius (Dirac: its box is one pixel) or with
-// one past 1e8 px keeps the whole box.  Rounded operations only, so that the
-// counts and the list agree whatever the compiler fuses.
+// 5.7 ms), 20 % on 500k wide ones in 1024^2 x 256 (30.4 to 25.8 ms).  `reach2`
+// is the squared radius in px with a margin far above the rounding of the FP32
+// weights (2e-5 relative and 2e-4 px); a kernel without a radius (Dirac: its box
+// is one pixel) or with one past 1e8 px keeps the whole box.  Rounded operations
+// only, so that the counts and the list agree whatever the compiler fuses.
 __device__ __forceinline__ float reach2(const PRec& r, const KSpec& k) {
   if (k.type == MG_KERNEL_DIRAC) return 1e30f;
   const float rad = k.type == MG_KERNEL_GAUSSIAN

@@ -33,7 +33,12 @@
 #include "mg_internal.cuh"
 
 namespace mg {
-void set_last_error(const std::string& msg);  // mg_api.cu
+// mg_api.cu
+void set_last_error(const std::string& msg);
+int workspace_size_small(const mg_problem* p, long long max_pairs, long long max_partial,
+                         size_t* bytes);
+int insert_small(const mg_problem* p, void* ws, size_t bytes, long long max_pairs,
+                 long long max_partial, cudaStream_t s);
 }
 
 namespace {
@@ -69,7 +74,7 @@ extern "C" int mg_insert_noalloc(const mg_problem* p, void* stream) {
   // capacities that fit the array: a quarter of what is left after the fixed
   // part goes to split-K partial tiles, the rest to the (tile, particle) list
   size_t fixed = 0;
-  rc = mg_workspace_size(p, 0, 0, &fixed);
+  rc = mg::workspace_size_small(p, 0, 0, &fixed);
   if (rc) return rc;
   if (fixed > cap) {
     mg::set_last_error("mg_insert_noalloc: problem too large for the built-in scratch (" +
@@ -78,9 +83,9 @@ extern "C" int mg_insert_noalloc(const mg_problem* p, void* stream) {
     return MG_ERR_WORKSPACE;
   }
   size_t one_partial = 0, one_partial0 = 0;
-  rc = mg_workspace_size(p, 0, 1, &one_partial);
+  rc = mg::workspace_size_small(p, 0, 1, &one_partial);
   if (rc) return rc;
-  rc = mg_workspace_size(p, 0, 0, &one_partial0);
+  rc = mg::workspace_size_small(p, 0, 0, &one_partial0);
   if (rc) return rc;
   const size_t partial_bytes = one_partial > one_partial0 ? one_partial - one_partial0 : 1;
   long long cap_partial = (long long)((cap - fixed) / 4 / partial_bytes);
@@ -89,11 +94,12 @@ extern "C" int mg_insert_noalloc(const mg_problem* p, void* stream) {
   while (hi - lo > 1) {
     const long long mid = lo + (hi - lo) / 2;
     size_t b = 0;
-    rc = mg_workspace_size(p, mid, cap_partial, &b);
+    rc = mg::workspace_size_small(p, mid, cap_partial, &b);
     if (rc) return rc;
     if (b <= cap) lo = mid; else hi = mid;
   }
-  rc = mg_insert(p, ws, MG_NOALLOC_SCRATCH_BYTES, lo, cap_partial, stream);
+  rc = mg::insert_small(p, ws, MG_NOALLOC_SCRATCH_BYTES, lo, cap_partial,
+                        static_cast<cudaStream_t>(stream));
   if (rc) return rc;
   rc = mg_check(ws, stream);
   if (rc == MG_ERR_WORKSPACE)

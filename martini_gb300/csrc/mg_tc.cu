@@ -58,9 +58,16 @@ constexpr int TC_DRAIN = 2;
 constexpr int KT_SMEM_CELLS = 1025;
 constexpr int TC_MASTER_COL = 256;
 // 64-particle stages of the three-piece split keep a second working
-// accumulator here (blocks of at most 128 channels): K-steps 0-1 accumulate
-// at column 0, K-steps 2-3 at this column, so each sees the MMA sequence of
-// a 32-particle stage before the drain
+// accumulator here: K-steps 0-1 accumulate at column 0, K-steps 2-3 at this
+// column, so each sees the MMA sequence of a 32-particle stage before the
+// drain.  Both hold the stage's window from its first channel on, so that only
+// the window is limited to 128 channels and the block is as wide as the master
+// (256): a line that straddles two 128-channel blocks would make two pairs
+// (1M particles in 512^2 x 256: 17.3M pairs with blocks of 128, 13.2M with 256,
+// contraction 5.75 ms and 4.67 ms; 500k wide ones in 1024^2 x 256: 25.8 ms and
+// 19.1 ms; 4M in 1024^2 x 512 whose lines hardly straddle: 6.50 and 6.70 ms).  A
+// stage whose window is wider (at a class boundary, or with few particles in
+// the segment) is taken in parts, its weights computed again for each.
 constexpr int TC_WB_COL = 128;
 
 // Operand splits: a hi + lo pair of FP16 (scaled) or BF16 pieces, or three
@@ -71,7 +78,7 @@ constexpr int SPLIT_BF16_3 = 2;
 __host__ __device__ constexpr int split_parts(int split) { return split == SPLIT_BF16_3 ? 3 : 2; }
 __host__ __device__ constexpr bool split_bf16(int split) { return split != SPLIT_F16_2; }
 // Particles per stage: 64 by default, 32 as a launch-shape choice.  The
-// three-piece split's 64-particle stages fit with blocks of 128 channels.
+// three-piece split's 64-particle stages fit with stage windows of 128 channels.
 
 // Shared memory at the widest band: two stages of A and B pieces plus the
 // static arrays must fit in the 227 KB of a CTA.
@@ -1206,8 +1213,7 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
   auto zero_tmem = [&](int lo, int hi) {
     for (int c = colgrp * 32; c < ncols; c += 128) {
       if (!chunk_in(c, lo, hi)) continue;
-      tmem_st32_zero(tmem + lane_base + c);
-      if (TWO_ACC) tmem_st32_zero(tmem + lane_base + TC_WB_COL + c);
+      if (!TWO_ACC) tmem_st32_zero(tmem + lane_base + c);
       if (drain) tmem_st32_zero(tmem + lane_base + TC_MASTER_COL + c);
     }
     tmem_wait_st();
@@ -1223,16 +1229,17 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
     if (colgrp >= dwarps) return;
     for (int c = (lo & ~15) + 16 * colgrp; c < hi; c += 16 * dwarps) {
       unsigned a[16], b[16];
-      tmem_ld16(tmem + lane_base + c, a);
+      const int wc = TWO_ACC ? c - lo : c;  // column of the working accumulator
+      tmem_ld16(tmem + lane_base + wc, a);
       tmem_ld16(tmem + lane_base + TC_MASTER_COL + c, b);
       if constexpr (TWO_ACC) {
         unsigned a2[16];
-        tmem_ld16(tmem + lane_base + TC_WB_COL + c, a2);
+        tmem_ld16(tmem + lane_base + TC_WB_COL + wc, a2);
         tmem_wait_ld();
 #pragma unroll
         for (int v = 0; v < 16; ++v)
           a[v] = __float_as_uint(__uint_as_float(a[v]) + __uint_as_float(a2[v]));
-        tmem_st16_zero(tmem + lane_base + TC_WB_COL + c);
+        tmem_st16_zero(tmem + lane_base + TC_WB_COL + wc);
       } else {
         tmem_wait_ld();
       }
@@ -1240,11 +1247,16 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
       for (int v = 0; v < 16; ++v)
         b[v] = __float_as_uint(__uint_as_float(a[v]) + __uint_as_float(b[v]));
       tmem_st16(tmem + lane_base + TC_MASTER_COL + c, b);
-      tmem_st16_zero(tmem + lane_base + c);
+      tmem_st16_zero(tmem + lane_base + wc);
     }
     tmem_wait_st();
   };
   zero_tmem(0, ncols);
+  if (TWO_ACC) {  // window-relative: cleared by the drains and the epilogue from here on
+    tmem_st32_zero(tmem + lane_base + colgrp * 32);
+    tmem_st32_zero(tmem + lane_base + TC_WB_COL + colgrp * 32);
+    tmem_wait_st();
+  }
   tc_fence_before();
   __syncthreads();
 
@@ -1315,7 +1327,10 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
     }
     __syncthreads();
 
-    for (int ch = 0; ch < nchunk; ++ch) {
+    int l_lo = 0, l_hi = 0;  // window of the last stage
+    // v counts the stages as issued: stage ch of the item, part `sub` of its
+    // window
+    for (int v = 0, ch = 0, sub = 0; ch < nchunk; ++v) {
       const int buf = ch % 3;              // this stage's parameters
       const int nbuf = buf == 2 ? 0 : buf + 1;  // the next stage's
       const int k0 = ch * KC;
@@ -1328,29 +1343,13 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
       }
       // the stage's parameters: built at the item's start for its first
       // stage, else by the build warps during the previous stage
-      if (ch > 0) {
+      if (ch > 0 && sub == 0) {
         if (!mbar_wait(smem_u32(&s_parb[buf]), (parb_par >> buf) & 1u)) s_abort = 1;
         parb_par ^= 1u << buf;
       }
-      // the next stage's records travel global -> shared by cp.async while
-      // this one is produced (its list entry was read a stage earlier); the
-      // list entry of the stage after is read now
-      const bool has_next = ch + 1 < nchunk;
-      int npid = 0;
-      if (has_next && bld) {
-        if (k0 + KC + bq < it.lcount) {
-          npid = pid_ahead;
-          cp_async_tpar(&s_tp[0][bq], KC * 16u, w.tpar + npid);
-        } else {
-          const TcPar z = empty_tpar();
-#pragma unroll
-          for (int k = 0; k < 4; ++k) s_tp[k][bq] = reinterpret_cast<const uint4*>(&z)[k];
-        }
-        cp_async_commit();
-        if (k0 + 2 * KC + bq < it.lcount) pid_ahead = w.list[it.lbeg + k0 + 2 * KC + bq];
-      }
       // stage channel window [w0, w0 + nw): min clo, max chi
       int w0, nw;
+      bool fin;  // the last part
       {
         // the extremes of the stage's listed particles' supports
         int2 lh = s_win[buf][0];
@@ -1363,16 +1362,33 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
         lo = max(lo, it.c0) - it.c0;
         hi = min(hi, it.c0 + ncols - 1) - it.c0;
         if (hi < lo) lo = hi = 0;  // no support in this block: zeros
-        w0 = lo & ~15;
-        nw = ((hi + 1 - w0) + 15) & ~15;
-        if (nw < 16) nw = 16;
-        if (nw > nwmax) nw = nwmax;
-        if (w0 + nw > ncols) w0 = ncols - nw;
-        if (w0 < 0) w0 = 0;
+        w0 = (lo & ~15) + (TWO_ACC ? sub * nwmax : 0);
+        const int end = (hi + 16) & ~15;  // at most ncols
+        fin = !TWO_ACC || end - w0 <= nwmax;
+        nw = fin ? end - w0 : nwmax;
+        l_lo = w0;
+        l_hi = w0 + nw;
         d_lo = min(d_lo, w0);
         d_hi = max(d_hi, w0 + nw);
         t_lo = min(t_lo, w0);
         t_hi = max(t_hi, w0 + nw);
+      }
+      // the next stage's records travel global -> shared by cp.async while
+      // this one is produced (its list entry was read a stage earlier); the
+      // list entry of the stage after is read now
+      const bool has_next = fin && ch + 1 < nchunk;
+      int npid = 0;
+      if (has_next && bld) {
+        if (k0 + KC + bq < it.lcount) {
+          npid = pid_ahead;
+          cp_async_tpar(&s_tp[0][bq], KC * 16u, w.tpar + npid);
+        } else {
+          const TcPar z = empty_tpar();
+#pragma unroll
+          for (int k = 0; k < 4; ++k) s_tp[k][bq] = reinterpret_cast<const uint4*>(&z)[k];
+        }
+        cp_async_commit();
+        if (k0 + 2 * KC + bq < it.lcount) pid_ahead = w.list[it.lbeg + k0 + 2 * KC + bq];
       }
       unsigned char* const sa = smem + stage * st_bytes;  // NP pieces of A, then of B
       unsigned char* const sb = sa + NP * a_bytes;
@@ -1444,7 +1460,7 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
         // the next stage's buffer of parameters was last read two stages
         // ago: every warp must have finished that stage (s_full[stage]'s
         // phase before the current one)
-        if (ch > 1 &&
+        if (v > 1 &&
             !mbar_wait(smem_u32(&s_full[stage]), ((full_par >> stage) & 1u) ^ 1u))
           s_abort = 1;
         s_pid[nbuf][bq] = npid;
@@ -1490,7 +1506,7 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
         const unsigned long long b_hi = sdesc(base + NP * a_bytes, 128, 256);
         const unsigned long long b_2 = b_hi + (b_bytes >> 4);
         const unsigned bstep = (unsigned)nw * 2u;  // K step of B: nw * 32 bytes
-        const unsigned d = tmem + (unsigned)w0;
+        const unsigned d = TWO_ACC ? tmem : tmem + (unsigned)w0;
         // Smallest terms first: the tensor core's FP32 accumulation truncates
         // each MMA's sum to the accumulator's precision, so every MMA loses up
         // to an ulp of the accumulator.  Issued into the working accumulator
@@ -1525,7 +1541,14 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
       if (s_abort) break;
       pending_bits |= 1u << stage;
       stage ^= 1;
-      if (drain && ++since_drain == DRAIN_STAGES && ch + 1 < nchunk) {
+      const bool more = !fin || ch + 1 < nchunk;
+      if (fin) {
+        ++ch;
+        sub = 0;
+      } else {
+        ++sub;
+      }
+      if (drain && ++since_drain == DRAIN_STAGES && more) {
         // drain the interval's columns during the next stage (its commit
         // covers every earlier MMA)
         drain_due = true;
@@ -1578,16 +1601,27 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
 #pragma unroll
           for (int v = 0; v < 32; ++v) r[v] = 0u;
         } else {
-          tmem_ld32(tmem + lane_base + (unsigned)c, r);
-          tmem_wait_ld();
-          if (TWO_ACC) {
+          if (!TWO_ACC) {
+            tmem_ld32(tmem + lane_base + (unsigned)c, r);
+            tmem_wait_ld();
+          } else {
+            // the last stage's window, not drained yet
             for (int h = 0; h < 32; h += 16) {
-              unsigned m[16];
-              tmem_ld16(tmem + lane_base + TC_WB_COL + (unsigned)(c + h), m);
-              tmem_wait_ld();
+              if (c + h >= l_lo && c + h < l_hi) {
+                unsigned a[16], m[16];
+                tmem_ld16(tmem + lane_base + (unsigned)(c + h - l_lo), a);
+                tmem_ld16(tmem + lane_base + TC_WB_COL + (unsigned)(c + h - l_lo), m);
+                tmem_wait_ld();
+                // read by this warp alone: cleared here for the next item
+                tmem_st16_zero(tmem + lane_base + (unsigned)(c + h - l_lo));
+                tmem_st16_zero(tmem + lane_base + TC_WB_COL + (unsigned)(c + h - l_lo));
 #pragma unroll
-              for (int v = 0; v < 16; ++v)
-                r[h + v] = __float_as_uint(__uint_as_float(r[h + v]) + __uint_as_float(m[v]));
+                for (int v = 0; v < 16; ++v)
+                  r[h + v] = __float_as_uint(__uint_as_float(a[v]) + __uint_as_float(m[v]));
+              } else {
+#pragma unroll
+                for (int v = 0; v < 16; ++v) r[h + v] = 0u;
+              }
             }
           }
           if (drain) {
@@ -1719,6 +1753,8 @@ __global__ void k_tc_params(Geo g, Ws w) {
 int launch_contract_bf16x3(const Geo& g, const Ws& w, int num_sms, cudaStream_t s) {
   const int nwmax = g.max_width;  // a stage window never exceeds the widest block
   if (nwmax > TC_MASTER_COL) return MG_ERR_UNSUPPORTED;
+  // windows of the two-accumulator stages: 128 channels at most
+  const int nw2 = nwmax < TC_WB_COL ? nwmax : TC_WB_COL;
   if (g.n > 0) {
     const unsigned blocks =
         (unsigned)std::min<long long>((g.n + 255) / 256, (long long)num_sms * 16);
@@ -1728,10 +1764,8 @@ int launch_contract_bf16x3(const Geo& g, const Ws& w, int num_sms, cudaStream_t 
   const bool kc32 = g.kc == 32;
   int rc;
   if (g.form == MG_FORM_BF16X6) {
-    // 64-particle stages hold two working accumulators of 128 columns
-    if (!kc32 && nwmax > TC_WB_COL) return MG_ERR_UNSUPPORTED;
     rc = kc32 ? launch_tc<SPLIT_BF16_3, 32>(g, w, num_sms, s, nwmax)
-              : launch_tc<SPLIT_BF16_3, 64>(g, w, num_sms, s, nwmax);
+              : launch_tc<SPLIT_BF16_3, 64>(g, w, num_sms, s, nw2);
   }
   else if (g.form == MG_FORM_BF16X3)
     rc = kc32 ? launch_tc<SPLIT_BF16_2, 32>(g, w, num_sms, s, nwmax)
