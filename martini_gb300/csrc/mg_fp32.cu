@@ -180,6 +180,7 @@ k_contract_fp32(Geo g, Ws w) {
     } else {
       const long long slot = w.part_off[it.seg] + it.kc;
       float* dst = w.partial + slot * (long long)(TILE_PX * g.max_width);
+      if (tid == 0) w.item_key[w.item_order[item]] = part_window(0, CBLK);
 #pragma unroll
       for (int a = 0; a < 8; ++a) {
         const int px = tr * 8 + a;
@@ -191,66 +192,90 @@ k_contract_fp32(Geo g, Ws w) {
 }
 
 // Split-K reduction, shared by every form: a segment with nk > 1 work items
-// left nk partial rows of TILE_PX x seg_width floats (pixel-major).  One
-// block per (segment, chunk of RED_CHUNK floats): each thread sums four
-// channels of one pixel over the rows in ascending row order, so the result
-// does not depend on scheduling, with RED_ROWS float4 loads in flight.
+// left nk partial rows of TILE_PX x seg_width floats (pixel-major), of which
+// an item wrote the channels of its window only (item_key, part_window).  A
+// block takes one chunk of RED_CHUNK floats of the split segments among
+// RED_SEGS: its lanes look them up at once, because few segments are split
+// and a block that visited every (segment, chunk) alone spent its time on
+// the lookups (4M particles in 1024^2 x 512: 0.45 ms, 0.04 ms now).  The RED_SEGS
+// lie a grid's length apart, so that dense neighbouring tiles go to different
+// blocks.  Each thread sums four channels of one pixel over the rows in
+// ascending row order, so the result does not depend on scheduling, with
+// RED_ROWS float4 loads in flight.
 constexpr int RED_THREADS = 256;
 constexpr int RED_CHUNK = RED_THREADS * 4;
 constexpr int RED_ROWS = 8;
+constexpr int RED_SEGS = 32;
+
+__device__ __forceinline__ void reduce_chunk(const Geo& g, const Ws& w, int sg, int nk,
+                                             int chunk) {
+  const long long slot = (long long)TILE_PX * g.max_width;  // floats per partial row
+  const int gk = find_gal(w.gs0, g.ngal, sg);
+  const Gal& G = w.gal[gk];
+  const int width = G.width;  // a multiple of 16 channels
+  const int e = chunk * RED_CHUNK + threadIdx.x * 4;
+  if (e >= TILE_PX * width) return;
+  const int px = e / width, cl = e - px * width;
+  const unsigned* win = w.item_key + w.item_off[sg];
+  const float4* src = reinterpret_cast<const float4*>(w.partial + w.part_off[sg] * slot + e);
+  const long long row4 = slot / 4;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k0 = 0; k0 < nk; k0 += RED_ROWS) {
+    float4 v[RED_ROWS];
+#pragma unroll
+    for (int q = 0; q < RED_ROWS; ++q)
+      if (k0 + q < nk) {
+        const unsigned pw = win[k0 + q];  // the row's channels [low half, high half)
+        v[q] = (unsigned)cl - (pw & 0xFFFFu) < (pw >> 16) - (pw & 0xFFFFu)
+                   ? __ldcs(src + (long long)(k0 + q) * row4)
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+    for (int q = 0; q < RED_ROWS; ++q)
+      if (k0 + q < nk) {
+        acc.x += v[q].x;
+        acc.y += v[q].y;
+        acc.z += v[q].z;
+        acc.w += v[q].w;
+      }
+  }
+  const int ls = sg - G.seg0;
+  const int t = ls / G.ncb;
+  const int cb = ls - t * G.ncb;
+  const int tx = t / G.nty, ty = t - tx * G.nty;
+  const int c = cb * width + cl;
+  const int i = tx * TILE_I + px / TILE_J, j = ty * TILE_J + px % TILE_J;
+  if (i >= G.nx || j >= G.ny) return;
+  const int nc = G.nc;
+  float* dst = G.cube + ((long long)i * G.ny + j) * nc + c;
+  if (g.accumulate) {
+    if (c < nc) acc.x += dst[0];
+    if (c + 1 < nc) acc.y += dst[1];
+    if (c + 2 < nc) acc.z += dst[2];
+    if (c + 3 < nc) acc.w += dst[3];
+  }
+  if (c < nc) dst[0] = acc.x;
+  if (c + 1 < nc) dst[1] = acc.y;
+  if (c + 2 < nc) dst[2] = acc.z;
+  if (c + 3 < nc) dst[3] = acc.w;
+}
 
 __global__ void __launch_bounds__(RED_THREADS) k_reduce_partials(Geo g, Ws w) {
   if (w.hdr->status) return;
-  const long long slot = (long long)TILE_PX * g.max_width;  // floats per partial row
-  const int nchunk = (int)((slot + RED_CHUNK - 1) / RED_CHUNK);
-  const long long units = (long long)g.nseg * nchunk;
+  const int nchunk = (TILE_PX * g.max_width + RED_CHUNK - 1) / RED_CHUNK;
+  const int ngrp = (g.nseg + RED_SEGS - 1) / RED_SEGS;
+  const long long units = (long long)ngrp * nchunk;
+  const int lane = threadIdx.x & 31;
   for (long long u = blockIdx.x; u < units; u += gridDim.x) {
-    const int sg = (int)(u / nchunk);
-    const int nk = w.seg_part[sg];
-    if (nk == 0) continue;
-    const int gk = find_gal(w.gs0, g.ngal, sg);
-    const Gal& G = w.gal[gk];
-    const int width = G.width;  // a multiple of 16 channels
-    const int per_row = TILE_PX * width;
-    const int e = (int)(u - (long long)sg * nchunk) * RED_CHUNK + threadIdx.x * 4;
-    if (e >= per_row) continue;
-    const float4* src =
-        reinterpret_cast<const float4*>(w.partial + w.part_off[sg] * slot + e);
-    const long long row4 = slot / 4;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k0 = 0; k0 < nk; k0 += RED_ROWS) {
-      float4 v[RED_ROWS];
-#pragma unroll
-      for (int q = 0; q < RED_ROWS; ++q)
-        if (k0 + q < nk) v[q] = __ldcs(src + (long long)(k0 + q) * row4);
-#pragma unroll
-      for (int q = 0; q < RED_ROWS; ++q)
-        if (k0 + q < nk) {
-          acc.x += v[q].x;
-          acc.y += v[q].y;
-          acc.z += v[q].z;
-          acc.w += v[q].w;
-        }
+    const int grp = (int)(u / nchunk), chunk = (int)(u - (long long)grp * nchunk);
+    const long long mine = grp + (long long)lane * ngrp;
+    const int nk = mine < g.nseg ? w.seg_part[mine] : 0;
+    for (unsigned m = __ballot_sync(0xffffffffu, nk > 0); m; m &= m - 1) {
+      const int l = __ffs(m) - 1;
+      const int n = __shfl_sync(0xffffffffu, nk, l);
+      reduce_chunk(g, w, grp + l * ngrp, n, chunk);
+      __syncwarp();
     }
-    const int ls = sg - G.seg0;
-    const int t = ls / G.ncb;
-    const int cb = ls - t * G.ncb;
-    const int tx = t / G.nty, ty = t - tx * G.nty;
-    const int px = e / width, c = cb * width + (e - px * width);
-    const int i = tx * TILE_I + px / TILE_J, j = ty * TILE_J + px % TILE_J;
-    if (i >= G.nx || j >= G.ny) continue;
-    const int nc = G.nc;
-    float* dst = G.cube + ((long long)i * G.ny + j) * nc + c;
-    if (g.accumulate) {
-      if (c < nc) acc.x += dst[0];
-      if (c + 1 < nc) acc.y += dst[1];
-      if (c + 2 < nc) acc.z += dst[2];
-      if (c + 3 < nc) acc.w += dst[3];
-    }
-    if (c < nc) dst[0] = acc.x;
-    if (c + 1 < nc) dst[1] = acc.y;
-    if (c + 2 < nc) dst[2] = acc.z;
-    if (c + 3 < nc) dst[3] = acc.w;
   }
 }
 

@@ -240,7 +240,9 @@ struct Ws {
   long long cap_spec;    // room in spec (the workspace beyond the fixed layout)
   // Work queue order: item_order[k] is the k-th item the contraction takes,
   // the items sorted by estimated cost, largest first (stable: equal costs
-  // keep segment order).  item_key / item_*_tmp are the sort's buffers.
+  // keep segment order).  item_key / item_*_tmp are the sort's buffers;
+  // from the contraction on, item_key[item] of a split segment's item is the
+  // part_window of its partial row.
   int* item_order;       // [cap_items]
   unsigned* item_key;    // [cap_items]
   unsigned* item_key_tmp;
@@ -281,6 +283,13 @@ void launch_order_particles(const Geo& g, const Ws& w, int* out, long long max_c
 int launch_contract_fp32(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
 int launch_contract_bf16x3(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
 void launch_reduce_partials(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
+
+// The channels [lo, hi) of its block that an item wrote in its partial row
+// (multiples of 16, at most 256), packed.
+__device__ __forceinline__ unsigned part_window(int lo, int hi) {
+  return (unsigned)lo | (unsigned)hi << 16;
+}
+
 void launch_spec_store(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
 void launch_flux_batch(const Geo& g, const Ws& w, cudaStream_t s);
 void launch_flux(const float* cube, int nx, int ny, int nc, int padx, int pady, double* part,

@@ -1592,47 +1592,46 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
         dst = w.partial + slot * (long long)(TILE_PX * g.max_width) + (long long)p * ncols;
         limit = ncols;
         vec = true;
+        if (tid == 0)
+          w.item_key[w.item_off[it.seg] + it.kc] =
+              part_window(t_lo & ~31, min((t_hi + 31) & ~31, ncols));
       }
       for (int c = colgrp * 32; c < ncols; c += 128) {
         unsigned r[32];
-        if (!chunk_in(c, t_lo, t_hi)) {
-          // never written: zero (already in a cleared or accumulated cube)
-          if (it.nk == 1) continue;
-#pragma unroll
-          for (int v = 0; v < 32; ++v) r[v] = 0u;
+        // never written: zero (already in a cleared or accumulated cube, and
+        // outside the window the reduction reads of a partial row)
+        if (!chunk_in(c, t_lo, t_hi)) continue;
+        if (!TWO_ACC) {
+          tmem_ld32(tmem + lane_base + (unsigned)c, r);
+          tmem_wait_ld();
         } else {
-          if (!TWO_ACC) {
-            tmem_ld32(tmem + lane_base + (unsigned)c, r);
-            tmem_wait_ld();
-          } else {
-            // the last stage's window, not drained yet
-            for (int h = 0; h < 32; h += 16) {
-              if (c + h >= l_lo && c + h < l_hi) {
-                unsigned a[16], m[16];
-                tmem_ld16(tmem + lane_base + (unsigned)(c + h - l_lo), a);
-                tmem_ld16(tmem + lane_base + TC_WB_COL + (unsigned)(c + h - l_lo), m);
-                tmem_wait_ld();
-                // read by this warp alone: cleared here for the next item
-                tmem_st16_zero(tmem + lane_base + (unsigned)(c + h - l_lo));
-                tmem_st16_zero(tmem + lane_base + TC_WB_COL + (unsigned)(c + h - l_lo));
-#pragma unroll
-                for (int v = 0; v < 16; ++v)
-                  r[h + v] = __float_as_uint(__uint_as_float(a[v]) + __uint_as_float(m[v]));
-              } else {
-#pragma unroll
-                for (int v = 0; v < 16; ++v) r[h + v] = 0u;
-              }
-            }
-          }
-          if (drain) {
-            for (int h = 0; h < 32; h += 16) {
-              unsigned m[16];
-              tmem_ld16(tmem + lane_base + TC_MASTER_COL + (unsigned)(c + h), m);
+          // the last stage's window, not drained yet
+          for (int h = 0; h < 32; h += 16) {
+            if (c + h >= l_lo && c + h < l_hi) {
+              unsigned a[16], m[16];
+              tmem_ld16(tmem + lane_base + (unsigned)(c + h - l_lo), a);
+              tmem_ld16(tmem + lane_base + TC_WB_COL + (unsigned)(c + h - l_lo), m);
               tmem_wait_ld();
+              // read by this warp alone: cleared here for the next item
+              tmem_st16_zero(tmem + lane_base + (unsigned)(c + h - l_lo));
+              tmem_st16_zero(tmem + lane_base + TC_WB_COL + (unsigned)(c + h - l_lo));
 #pragma unroll
               for (int v = 0; v < 16; ++v)
-                r[h + v] = __float_as_uint(__uint_as_float(r[h + v]) + __uint_as_float(m[v]));
+                r[h + v] = __float_as_uint(__uint_as_float(a[v]) + __uint_as_float(m[v]));
+            } else {
+#pragma unroll
+              for (int v = 0; v < 16; ++v) r[h + v] = 0u;
             }
+          }
+        }
+        if (drain) {
+          for (int h = 0; h < 32; h += 16) {
+            unsigned m[16];
+            tmem_ld16(tmem + lane_base + TC_MASTER_COL + (unsigned)(c + h), m);
+            tmem_wait_ld();
+#pragma unroll
+            for (int v = 0; v < 16; ++v)
+              r[h + v] = __float_as_uint(__uint_as_float(r[h + v]) + __uint_as_float(m[v]));
           }
         }
         if (inside || it.nk != 1) {
