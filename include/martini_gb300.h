@@ -373,6 +373,16 @@ int mg_flux(const float* cube, int32_t nx, int32_t ny, int32_t nc, int32_t padx,
             void* stream);
 
 /*
+ * An inserted cube into a caller's array, both in host memory and of shape
+ * [nx][ny][nc]: array = (array + add) / px2 with divide_all, else array +=
+ * add / px2 (martini/martini.py:358-366); per_channel[c] = sum of array px2
+ * over the pixels at least padx, pady from the edges, in a fixed order.
+ */
+int mg_cube_add(double* array, const float* add, int64_t nx, int64_t ny, int64_t nc,
+                int64_t padx, int64_t pady, double px2, int32_t divide_all,
+                double* per_channel);
+
+/*
  * Size of the scratch array built into the library for mg_insert_noalloc
  * (held on every GPU that loads the library until the process exits).
  */

@@ -27,6 +27,25 @@ FORMS = {"fp32": N.MG_FORM_FP32, "bf16x3": N.MG_FORM_BF16X3, "f16x3": N.MG_FORM_
 DEFAULT_FORM = "bf16x6"
 
 
+def add_to_array(array, add, pads, px2, divide_all):
+    """Add the FP32 cube ``add`` to the FP64 host ``array`` (its shape, or one
+    more axis of length 1) in one native pass: ``(array + add) / px2`` when
+    ``divide_all``, else ``array + add / px2``.  Returns the per-channel sums
+    of ``array * px2`` over the pixels inside ``pads``."""
+    if not array.flags.writeable:
+        raise ValueError("output array is read-only")
+    # a view (a cube without its pad) or another type goes through a copy
+    work = np.ascontiguousarray(array, dtype=np.float64)
+    add = np.ascontiguousarray(add, dtype=np.float32)
+    nx, ny, nc = add.shape
+    per_channel = np.empty(nc)
+    N.check(N.load().mg_cube_add(work.ctypes.data, add.ctypes.data, nx, ny, nc, *pads, float(px2),
+                                 int(divide_all), per_channel.ctypes.data))
+    if work is not array:
+        array[...] = work
+    return per_channel
+
+
 class _BaseMartini:
     def __init__(self, *, source, datacube: DataCube, beam=None, noise=None, sph_kernel,
                  spectral_model, quiet: bool = False, _prune_kwargs: dict | None = None,
@@ -103,7 +122,8 @@ class _BaseMartini:
         src, k, sm = self.source, self.sph_kernel, self.spectral_model
         h_eff, kidx = k._device_arrays()
         sig, sig_const = sm._device_sigma(src)
-        amp = src.mHI_g * np.power(src.skycoords.distance, -2.0) / MHI_TO_JY
+        d = np.asarray(src.skycoords.distance)
+        amp = src.mHI_g / (d * d) / MHI_TO_JY
         dev = self.engine.device
         parts = DeviceParticles.from_host(
             dev, src.pixcoords[0], src.pixcoords[1], k.sm_ranges, h_eff, kidx,
@@ -133,28 +153,19 @@ class _BaseMartini:
         nx, ny, nc = dc._array.shape[:3]
         cube, flux = self.engine.insert(parts, kernels, model, sig_const, nx, ny, nc, edges,
                                         padx=dc.padx, pady=dc.pady, form=FORMS[self.form])
-        add = cube.cpu().numpy().astype(np.float64)
-        flux = flux.cpu().numpy()
-        if dc.stokes_axis:
-            add = add[..., np.newaxis]
         px2 = dc.px_size**2
-        if dc._array_unit == "Jy/pix2":
-            dc._array += add
-            dc._array /= px2
-        else:
-            dc._array += add / px2
+        # the summary sums the whole converted array, prior contents
+        # included, over the unpadded pixels when both pads are non-zero
+        # (martini/martini.py:367-392)
+        pads = (dc.padx, dc.pady) if dc.padx > 0 and dc.pady > 0 else (0, 0)
+        per_channel = add_to_array(dc._array, cube.cpu().numpy(), pads, px2,
+                                   divide_all=dc._array_unit == "Jy/pix2")
+        flux = flux.cpu().numpy()
         dc._array_unit = "Jy/arcsec2"
         # this insertion's FP64 flux sums over the unpadded cube (total, then
         # per channel), from the GPU
         self._last_flux = flux
-        # the summary sums the whole converted array, prior contents
-        # included, over the unpadded pixels when both pads are non-zero
-        # (martini/martini.py:367-392)
-        pad_mask = (np.s_[dc.padx:-dc.padx, dc.pady:-dc.pady, ...]
-                    if dc.padx > 0 and dc.pady > 0 else np.s_[...])
-        in_jy = dc._array[pad_mask] * px2
-        inserted_flux = float(np.sum(in_jy))
-        per_channel = in_jy.sum(axis=(0, 1)).reshape(-1)
+        inserted_flux = float(np.sum(per_channel))
         inserted_mass = MHI_TO_JY * self.source.distance**2 * float(
             np.sum(per_channel * np.abs(np.diff(dc.velocity_channel_edges))))
         self.inserted_flux_density = inserted_flux
