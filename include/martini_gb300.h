@@ -194,6 +194,15 @@ int mg_workspace_size_batched(const mg_problem* probs, int32_t nprob, int64_t ma
                               int64_t max_partial_items, size_t* bytes);
 int mg_plan_batched(const mg_problem* probs, int32_t nprob, void* workspace,
                     size_t workspace_bytes, void* stream, mg_plan_info* info);
+/*
+ * mg_insert that continues from the binning of mg_plan: the last call on this
+ * workspace must have been mg_plan of this problem (cube, flux and accumulate
+ * may differ), with the particles unchanged since.  A plan serves one run;
+ * without one, mg_check reports MG_ERR_INVALID_ARGUMENT and the cube is not
+ * written beyond its clearing.
+ */
+int mg_insert_planned(const mg_problem* p, void* workspace, size_t workspace_bytes,
+                      int64_t max_pairs, int64_t max_partial_items, void* stream);
 int mg_insert_batched(const mg_problem* probs, int32_t nprob, void* workspace,
                       size_t workspace_bytes, int64_t max_pairs, int64_t max_partial_items,
                       void* stream);

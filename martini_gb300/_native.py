@@ -46,7 +46,8 @@ EXPORTS = ("mg_version", "mg_last_error", "mg_workspace_size", "mg_plan", "mg_in
            "mg_insert_stages_batched", "mg_setup_workspace_size", "mg_setup",
            "mg_global_profile_workspace_size", "mg_global_profile", "mg_convolve_beam",
            "mg_tuning_default", "mg_tuning_candidates", "mg_tune", "mg_tune_batched",
-           "mg_tuning_lookup", "mg_tuning_store", "mg_tuning_reset", "mg_cube_add")
+           "mg_tuning_lookup", "mg_tuning_store", "mg_tuning_reset", "mg_cube_add",
+           "mg_insert_planned")
 
 MG_NOALLOC_SCRATCH_BYTES = 128 << 20
 
@@ -155,6 +156,7 @@ def load(path: str = LIB_PATH) -> C.CDLL:
                               C.c_void_p]
     lib.mg_insert_stages.argtypes = [P(Problem), C.c_void_p, C.c_size_t, C.c_int64, C.c_int64,
                                      C.c_int32, C.c_void_p]
+    lib.mg_insert_planned.argtypes = lib.mg_insert.argtypes
     lib.mg_check.argtypes = [C.c_void_p, C.c_void_p]
     lib.mg_workspace_size_batched.argtypes = [P(Problem), C.c_int32, C.c_int64, C.c_int64,
                                               P(C.c_size_t)]
@@ -195,7 +197,8 @@ def load(path: str = LIB_PATH) -> C.CDLL:
               "mg_spectra", "mg_flux", "mg_insert_noalloc", "mg_workspace_size_batched",
               "mg_plan_batched", "mg_insert_batched", "mg_insert_stages_batched", "mg_setup",
               "mg_global_profile", "mg_convolve_beam", "mg_tuning_candidates", "mg_tune",
-              "mg_tune_batched", "mg_tuning_lookup", "mg_tuning_store", "mg_cube_add"):
+              "mg_tune_batched", "mg_tuning_lookup", "mg_tuning_store", "mg_cube_add",
+              "mg_insert_planned"):
         getattr(lib, f).restype = C.c_int
     _lib = lib
     return lib

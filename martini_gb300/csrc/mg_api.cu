@@ -467,11 +467,30 @@ std::string class_key(const Batch& b, long long max_pairs) {
   return k;
 }
 
+// What a plan depends on, as a 64-bit hash (FNV-1a) that is never 0.
+unsigned long long plan_key(const mg_problem* probs, int nprob) {
+  unsigned long long h = 14695981039346656037ull;
+  auto mix = [&](const void* v, size_t bytes) {
+    const unsigned char* b = static_cast<const unsigned char*>(v);
+    for (size_t k = 0; k < bytes; ++k) h = (h ^ b[k]) * 1099511628211ull;
+  };
+  auto add = [&](auto... v) { (mix(&v, sizeof(v)), ...); };
+  add(nprob);
+  for (int k = 0; k < nprob; ++k) {
+    const mg_problem& p = probs[k];
+    add(p.n, p.x, p.y, p.sm_range, p.h_eff, p.kernel_index, p.n_kernels, p.spectral_model, p.v,
+        p.sigma, p.sigma_const, p.amp, p.spectra, p.nx, p.ny, p.nc, p.padx, p.pady, p.edges,
+        p.form);
+    for (int j = 0; j < p.n_kernels; ++j) add(p.kernels[j].type, p.kernels[j].truncate);
+  }
+  return h ? h : 1ull;
+}
+
 // The stages of an insertion (MG_STAGE_* bits; `scatter` adds the particle
 // list to the binning stage); all asynchronous on stream s.
 int run(const mg_problem* probs, int nprob, void* ws, size_t bytes, cudaStream_t s,
         long long cap_pairs, long long cap_partial, int stages, bool scatter, Ws* wout,
-        Batch* bout, const mg_tuning* shape, bool small_partials = false) {
+        Batch* bout, const mg_tuning* shape, bool small_partials = false, bool resume = false) {
   Batch& b = *bout;
   int rc = make_batch(probs, nprob, &b, false, small_partials);
   if (rc) return rc;
@@ -483,7 +502,11 @@ int run(const mg_problem* probs, int nprob, void* ws, size_t bytes, cudaStream_t
   if (rc) return rc;
   launch_set_gals(b.gal.data(), g, w, s);
   if (stages & MG_STAGE_BIN) {
-    launch_prep(g, w, num_sms(), s, cap_pairs, cap_partial);
+    if (resume)
+      launch_resume(g, w, num_sms(), s, cap_pairs, cap_partial, plan_key(probs, nprob));
+    else
+      launch_prep(g, w, num_sms(), s, cap_pairs, cap_partial,
+                  scatter ? 0 : plan_key(probs, nprob));
     if (scatter) launch_sort_segments(g, w, cap_pairs, num_sms(), s);
   }
   if ((stages & MG_STAGE_SPEC) && tc_form(g.form)) launch_spec_store(g, w, num_sms(), s);
@@ -591,6 +614,16 @@ int mg_insert_stages_batched(const mg_problem* probs, int32_t nprob, void* works
              max_pairs, max_partial_items, stages, true, &w, &b, &shape);
 }
 
+int mg_insert_planned(const mg_problem* p, void* workspace, size_t workspace_bytes,
+                      int64_t max_pairs, int64_t max_partial_items, void* stream) {
+  Ws w;
+  Batch b;
+  mg_tuning shape;
+  mg_tuning_lookup(p, 1, max_pairs, &shape);
+  return run(p, 1, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), max_pairs,
+             max_partial_items, MG_STAGE_ALL, true, &w, &b, &shape, false, true);
+}
+
 int mg_insert_batched(const mg_problem* probs, int32_t nprob, void* workspace,
                       size_t workspace_bytes, int64_t max_pairs, int64_t max_partial_items,
                       void* stream) {
@@ -619,6 +652,8 @@ int mg_check(void* workspace, void* stream) {
   if (e != cudaSuccess) return cuda_fail(e, "mg_check");
   if (h.status & ST_EDGES)
     return fail(MG_ERR_NOT_MONOTONIC, "Channel edges are not monotonic sequence.");
+  if (h.status & ST_NO_PLAN)
+    return fail(MG_ERR_INVALID_ARGUMENT, "mg_insert_planned: the workspace holds no plan of the problem");
   if (h.status & ST_TIMEOUT)
     return fail(MG_ERR_TIMEOUT, "a device-side pipeline wait expired (results invalid)");
   if (h.status)

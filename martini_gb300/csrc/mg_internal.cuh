@@ -176,6 +176,7 @@ constexpr unsigned ST_PAIRS = 1u;        // pairs exceed the list capacity
 constexpr unsigned ST_PARTIALS = 2u;     // split-K partials exceed capacity
 constexpr unsigned ST_EDGES = 4u;        // channel edges not strictly monotonic
 constexpr unsigned ST_TIMEOUT = 8u;      // a bounded device-side wait expired
+constexpr unsigned ST_NO_PLAN = 16u;     // no plan of the problem to continue from
 
 // Workspace header (device): status flags and scalar counters.
 struct WsHeader {
@@ -194,6 +195,7 @@ struct WsHeader {
   int spec_ready;                // 1 once the store holds this binning's spectra
   int kch;                       // particles per work item (item_particles)
   long long n_valid;             // particles with pairs (particle list stage)
+  unsigned long long plan_key;   // problem whose plan the workspace holds, 0: none
 };
 
 // Pointers into the workspace (host computes, passes by value).  Arrays run
@@ -262,7 +264,9 @@ __host__ __device__ inline long long items_bound(long long nseg, long long cap_p
 // Host-side launchers (all asynchronous on stream s).
 void launch_set_gals(const Gal* gals, const Geo& g, const Ws& w, cudaStream_t s);
 void launch_prep(const Geo& g, const Ws& w, int num_sms, cudaStream_t s, long long cap_pairs,
-                 long long cap_partial);
+                 long long cap_partial, unsigned long long plan_key);
+void launch_resume(const Geo& g, const Ws& w, int num_sms, cudaStream_t s, long long cap_pairs,
+                   long long cap_partial, unsigned long long plan_key);
 void launch_sort_segments(const Geo& g, const Ws& w, long long cap_pairs, int num_sms,
                           cudaStream_t s);
 int sort_bits(const Geo& g);

@@ -528,6 +528,7 @@ __device__ __forceinline__ void produce_s_pair(const PRec& r0, const PRec& r1, b
 // that reaches the cube (0 otherwise).  Written over the per-particle pair
 // counts, which the binning stage no longer needs.
 __global__ void k_spec_count(Geo g, Ws w) {
+  if (w.hdr->status & ST_NO_PLAN) return;  // no records
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < g.n;
        p += (long long)gridDim.x * blockDim.x) {
     const PRec& r = w.rec[p];
@@ -565,7 +566,7 @@ __device__ __forceinline__ SpecIn spec_in(const Ws& w, long long p) {
 __global__ void k_spec_eval(Geo g, Ws w) {
   const bool form_bf16 = g.form == MG_FORM_BF16X3;
   const bool form_fp32 = g.form == MG_FORM_BF16X6;  // the contraction splits the FP32 value
-  const bool fits = w.hdr->n_spec <= w.cap_spec;
+  const bool fits = w.hdr->n_spec <= w.cap_spec && !(w.hdr->status & ST_NO_PLAN);
   // read by the contraction, which runs after this whole kernel
   if (blockIdx.x == 0 && threadIdx.x == 0) w.hdr->spec_ready = fits ? 1 : 0;
   if (!fits) return;
@@ -1724,6 +1725,7 @@ void launch_spec_store(const Geo& g, const Ws& w, int num_sms, cudaStream_t s) {
 // store row (pair_off holds the store's row offsets after the SPEC stage).
 __global__ void k_tc_params(Geo g, Ws w) {
   __shared__ KSpec s_ks[MG_MAX_KERNELS];
+  if (w.hdr->status & ST_NO_PLAN) return;  // no records
   if (threadIdx.x < MG_MAX_KERNELS) s_ks[threadIdx.x] = g.ks[threadIdx.x];
   __syncthreads();
   int ktab_type = -1;

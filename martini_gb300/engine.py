@@ -67,6 +67,7 @@ class InsertionEngine:
         self.device = torch.device(device) if device is not None else torch.device(
             "cuda", torch.cuda.current_device())
         self._ws = None
+        self._binned = False  # the workspace holds the binning of the last plan
         self._caps = (0, 0)
         self.last_plan = None
 
@@ -112,8 +113,9 @@ class InsertionEngine:
         N.check(self.lib.mg_plan(C.byref(prob), C.c_void_p(ws.data_ptr()), ws.numel(),
                                  C.c_void_p(s.cuda_stream), C.byref(info)))
         self._caps = (int(info.n_pairs), int(info.n_partial_items))
-        # the plan's size includes the spectrum store of the tensor-core forms
-        self._workspace(int(info.workspace_bytes))
+        # the plan's size includes the spectrum store of the tensor-core forms;
+        # a workspace that had to grow no longer holds the binning
+        self._binned = self._workspace(int(info.workspace_bytes)) is ws
         self.last_plan = info
         return info
 
@@ -140,6 +142,16 @@ class InsertionEngine:
         ws = self._ws
         N.check(self.lib.mg_insert(C.byref(prob), C.c_void_p(ws.data_ptr()), ws.numel(),
                                    self._caps[0], self._caps[1], C.c_void_p(s.cuda_stream)))
+
+    def _run_planned(self, prob: N.Problem) -> None:
+        """:meth:`run` directly after :meth:`plan` of the same problem: continues
+        from the plan's binning where the workspace still holds it."""
+        if not self._binned:
+            return self.run(prob)
+        s = torch.cuda.current_stream(self.device)
+        N.check(self.lib.mg_insert_planned(C.byref(prob), C.c_void_p(self._ws.data_ptr()),
+                                           self._ws.numel(), self._caps[0], self._caps[1],
+                                           C.c_void_p(s.cuda_stream)))
 
     def capture(self, prob: N.Problem) -> "torch.cuda.CUDAGraph":
         """Capture mg_insert of ``prob`` (after :meth:`plan`) in a CUDA graph:
@@ -184,7 +196,9 @@ class InsertionEngine:
                             edges, cube, fl, form, accumulate)
         if plan or self._ws is None:
             self.plan(prob)
-        self.run(prob)
+            self._run_planned(prob)
+        else:
+            self.run(prob)
         if check:
             self.check()
         return cube, fl
