@@ -54,7 +54,7 @@ FORMS = {"fp32": 0, "bf16x3": 1, "f16x3": 2, "bf16x6": 3}
 TRAFFIC_BYTES = {("disc4m_1024", "bf16x6"): 5_896_006_400}
 
 
-def launches_per_step(form: str, gaussian: bool, nx: int, ny: int, nc: int, n: int, pairs: int,
+def launches_per_step(form: str, lines: bool, nx: int, ny: int, nc: int, n: int, pairs: int,
                       ngal: int = 1, ntiles: int | None = None, nseg: int | None = None) -> int:
     """Kernels one mg_insert(_batched) launches: cube table (one per 16
     cubes), tile init, edges, prep, pair scan, difference-array prefix, tile
@@ -84,7 +84,7 @@ def launches_per_step(form: str, gaussian: bool, nx: int, ny: int, nc: int, n: i
     k = (ngal + 15) // 16 + 1 + 1 + 1 + scan(n) + 1 + scan(ntiles) + 1
     k += dist(n, 9) + scan(n) + 1 + passes * dist(pairs, -(-bits // passes)) + 1
     k += 2 * scan(nseg) + 1 + dist(items, 9) + 1
-    if form != "fp32" and gaussian:
+    if form != "fp32" and lines:
         k += 1 + scan(n) + 1
     if form != "fp32":
         k += 1
@@ -540,7 +540,7 @@ def main():
         "e2e": {"value": 1.0 / t_e2e, "unit": "cubes/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h)},
         "gpu_launches": a.steps * sum(launches_per_step(
-            a.form, g["prob"].spectral_model == N.MG_SPECTRUM_GAUSSIAN, nx, ny, nc,
+            a.form, g["prob"].spectral_model != N.MG_SPECTRUM_TABLE, nx, ny, nc,
             int(g["prob"].n), int(g["info"].n_pairs)) for g in ins),
         "step_ms": [round(t * 1e3, 3) for t in t_step],
         "clocks": clk,

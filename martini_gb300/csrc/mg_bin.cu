@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(PREP_THREADS) k_prep(Geo g, Ws w, long long pe
   __syncthreads();
   if (lane == 0) atomicAdd(&s_spec, (unsigned long long)my_spec);
   __syncthreads();
-  if (threadIdx.x == 0 && g.spectral_model == MG_SPECTRUM_GAUSSIAN)
+  if (threadIdx.x == 0 && stored_lines(g.spectral_model))
     atomicAdd(reinterpret_cast<unsigned long long*>(&w.hdr->spec_bound), s_spec);
 }
 

@@ -288,6 +288,11 @@ int launch_contract_fp32(const Geo& g, const Ws& w, int num_sms, cudaStream_t s)
 int launch_contract_bf16x3(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
 void launch_reduce_partials(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
 
+// Spectral models whose lines the tensor-core forms keep per particle.
+__host__ __device__ inline bool stored_lines(int model) {
+  return model == MG_SPECTRUM_GAUSSIAN || model == MG_SPECTRUM_DIRAC;
+}
+
 // The channels [lo, hi) of its block that an item wrote in its partial row
 // (multiples of 16, at most 256), packed.
 __device__ __forceinline__ unsigned part_window(int lo, int hi) {
