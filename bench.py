@@ -84,7 +84,7 @@ def launches_per_step(form: str, lines: bool, nx: int, ny: int, nc: int, n: int,
     k = (ngal + 15) // 16 + 1 + 1 + 1 + scan(n) + 1 + scan(ntiles) + 1
     k += dist(n, 9) + scan(n) + 1 + passes * dist(pairs, -(-bits // passes)) + 1
     k += 2 * scan(nseg) + 1 + dist(items, 9) + 1
-    if form != "fp32" and lines:
+    if lines:
         k += 1 + scan(n) + 1
     if form != "fp32":
         k += 1

@@ -373,8 +373,8 @@ int workspace_view(const Geo& g, void* ws, size_t bytes, long long cap_pairs,
   *w = make_ws(ws, L);
   if (sort_bits(g) > 32) return fail(MG_ERR_INVALID_ARGUMENT, "cube too large for the sort key");
   // the workspace beyond the fixed layout holds the spectrum store of the
-  // tensor-core forms (not TABLE); without room they evaluate in-kernel
-  if (tc_form(g.form) && stored_lines(g.spectral_model)) {
+  // Gaussian and Dirac lines; without room they are evaluated in-kernel
+  if (stored_lines(g.spectral_model)) {
     w->spec = reinterpret_cast<unsigned*>(static_cast<char*>(ws) + L.total);
     w->cap_spec = (long long)((bytes - L.total) / sizeof(unsigned));
   }
@@ -509,7 +509,7 @@ int run(const mg_problem* probs, int nprob, void* ws, size_t bytes, cudaStream_t
                   scatter ? 0 : plan_key(probs, nprob));
     if (scatter) launch_sort_segments(g, w, cap_pairs, num_sms(), s);
   }
-  if ((stages & MG_STAGE_SPEC) && tc_form(g.form)) launch_spec_store(g, w, num_sms(), s);
+  if (stages & MG_STAGE_SPEC) launch_spec_store(g, w, num_sms(), s);
   cudaError_t e;
   if (stages & MG_STAGE_CONTRACT) {
     e = cudaSuccess;
@@ -588,7 +588,7 @@ int mg_plan_batched(const mg_problem* probs, int32_t nprob, void* workspace,
   info->n_partial_items = h.partial_bound;
   info->n_tiles = b.g.ntiles;
   size_t spec_bytes = 0;
-  if (tc_form(b.g.form) && stored_lines(b.g.spectral_model))
+  if (stored_lines(b.g.spectral_model))
     // one 32-bit word per support channel: packed hi | lo halves, or the FP32
     // value the three-piece BF16 split is taken from
     spec_bytes = align256(sizeof(unsigned) * (size_t)h.spec_bound);

@@ -34,6 +34,12 @@ void set_last_error(const std::string& msg);  // mg_api.cu
 
 namespace {
 
+using mg::f2;
+using mg::f2_add;
+using mg::f2_fma;
+using mg::f2_make;
+using mg::f2_split;
+
 constexpr int BT_I = 16;    // output rows per block, two per warp
 constexpr int BT_J = 16;    // output columns per thread
 constexpr int BC = 32;      // channels per block (one per lane)
@@ -47,30 +53,6 @@ __host__ __device__ inline int beam_kstride(int ky) { return (ky + 3) & ~3; }
 size_t beam_smem(int kx, int ky) {
   return sizeof(float) *
          ((size_t)BR_RING * (BT_J + ky - 1) * BC + 2 * (size_t)(kx + 1) * beam_kstride(ky));
-}
-
-// Two FP32 values in a register pair: one instruction does both FMAs (each
-// rounds as the scalar FMA does).
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 f2_make(float a, float b) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 f2_split(f2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
-  f2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
 }
 
 // Taps b0 .. b0 + T - 1 of a step's kernel-row pair kp[b] = (row of output row

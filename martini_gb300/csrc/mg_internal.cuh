@@ -288,7 +288,7 @@ int launch_contract_fp32(const Geo& g, const Ws& w, int num_sms, cudaStream_t s)
 int launch_contract_bf16x3(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
 void launch_reduce_partials(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
 
-// Spectral models whose lines the tensor-core forms keep per particle.
+// Spectral models whose lines are kept per particle (the spectrum store).
 __host__ __device__ inline bool stored_lines(int model) {
   return model == MG_SPECTRUM_GAUSSIAN || model == MG_SPECTRUM_DIRAC;
 }
@@ -436,6 +436,31 @@ __device__ __forceinline__ void channel_range(const double* e, int nc, int dec, 
     c0 = first;
     c1 = last;
   }
+}
+
+// Two FP32 values in a register pair: one instruction does both operations,
+// each rounded as the scalar one (the pipe takes as long as for two; the issue
+// slot is saved).
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 f2_make(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_split(f2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
 // ---------------------------------------------------------------------------

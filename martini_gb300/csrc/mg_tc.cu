@@ -626,6 +626,28 @@ __global__ void k_spec_eval(Geo g, Ws w) {
   }
 }
 
+// The FP32 form's lines, by its own line function (the same bits as lines
+// evaluated in the contraction), a warp per particle.
+__global__ void k_spec_fp32(Geo g, Ws w) {
+  const bool fits = w.hdr->n_spec <= w.cap_spec && !(w.hdr->status & ST_NO_PLAN);
+  if (blockIdx.x == 0 && threadIdx.x == 0) w.hdr->spec_ready = fits ? 1 : 0;
+  if (!fits) return;
+  const int lane = threadIdx.x & 31;
+  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long p = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; p < g.n;
+       p += nwarps) {
+    const int cnt = w.npairs[p];
+    if (cnt <= 0) continue;
+    const PRec r = w.rec[p];
+    const int gk = find_gal(w.gp0, g.ngal, p);
+    const int e0 = w.gal[gk].edge0, dec = w.gst[gk].dec;
+    unsigned* out = w.spec + w.pair_off[p];
+    for (int m = lane; m < cnt; m += 32)
+      out[m] = __float_as_uint(channel_spectrum(r, g.spectral_model, r.clo + m, dec, w.ehi + e0,
+                                                w.elo + e0, w.inv_w + e0));
+  }
+}
+
 // Dirac lines (one channel, two for a velocity on an edge), a thread per
 // particle.  Evaluated by the producer instead, every stage read 64 records
 // from global memory in the middle of its production (200k particles, 21.5M
@@ -1734,7 +1756,7 @@ int launch_tc(const Geo& g, const Ws& w, int num_sms, cudaStream_t s, int nwmax)
   return MG_OK;
 }
 
-// Spectrum store of the tensor-core forms (Gaussian and Dirac lines): row lengths,
+// Spectrum store (Gaussian and Dirac lines): row lengths,
 // their scan into row offsets, the rows.
 void launch_spec_store(const Geo& g, const Ws& w, int num_sms, cudaStream_t s) {
   const long long n = g.n;
@@ -1742,6 +1764,11 @@ void launch_spec_store(const Geo& g, const Ws& w, int num_sms, cudaStream_t s) {
   const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, (long long)num_sms * 16);
   k_spec_count<<<blocks, 256, 0, s>>>(g, w);
   launch_scan(w.npairs, n, w.pair_off, w.scan_sums, &w.hdr->n_spec, s);
+  if (g.form == MG_FORM_FP32) {
+    k_spec_fp32<<<(unsigned)std::min<long long>((n + 7) / 8, (long long)num_sms * 32), 256, 0, s>>>(
+        g, w);
+    return;
+  }
   if (g.spectral_model == MG_SPECTRUM_DIRAC) {
     k_spec_dirac<<<blocks, 256, 0, s>>>(g, w);
     return;
