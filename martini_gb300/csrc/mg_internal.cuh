@@ -38,7 +38,7 @@ __host__ __device__ inline int item_particles(long long total_pairs, int num_sms
 }
 
 // Per-particle record written by the prep kernel (64 bytes).
-struct PRec {
+struct __align__(8) PRec {
   int ilo, ihi, jlo, jhi;  // exact footprint box (inclusive), clipped; empty if ilo > ihi
   int xi, yi;              // floor(x), floor(y)
   float xf, yf;            // x - xi, y - yi in [0, 1)
@@ -336,12 +336,14 @@ struct AbsWithin {
 
 // Inclusive pixel range [lo, hi] of {i : |i - c| <= r}, clipped to [0, n).
 __device__ __forceinline__ void box_bounds(double c, double r, int n, int& lo, int& hi) {
-  if (!(r >= 0.0)) {  // NaN or negative range: empty
+  constexpr long long kInf = 0x7ff0000000000000ll;
+  const long long rb = __double_as_longlong(r);  // r >= 0: the bits order as the values
+  if (rb > kInf || (rb < 0 && rb != (long long)0x8000000000000000ull)) {  // NaN or negative: empty
     lo = 0;
     hi = -1;
     return;
   }
-  if (isinf(r)) {
+  if (rb == kInf) {
     lo = 0;
     hi = n - 1;
     return;
@@ -349,22 +351,27 @@ __device__ __forceinline__ void box_bounds(double c, double r, int n, int& lo, i
   const AbsWithin in(c, r);
   // scan start points outside the answer on both sides: FP32 for moderate
   // coordinates (off by < 0.2 there, so one extra step of margin), FP64 else
-  double a, b;
+  int l, h;
   if (in.fast) {
-    a = (double)(floorf(in.cf - in.rf) - 2.f);
-    b = (double)(ceilf(in.cf + in.rf) + 2.f);
+    l = max((int)floorf(in.cf - in.rf) - 2, 0);
+    h = min((int)ceilf(in.cf + in.rf) + 2, n - 1);
   } else {
-    a = floor(c - r) - 1.0;
-    b = ceil(c + r) + 1.0;
+    double a = floor(c - r) - 1.0, b = ceil(c + r) + 1.0;
+    if (a < 0.0) a = 0.0;
+    if (b > (double)(n - 1)) b = (double)(n - 1);
+    if (a > b) {
+      lo = 0;
+      hi = -1;
+      return;
+    }
+    l = (int)a;
+    h = (int)b;
   }
-  if (a < 0.0) a = 0.0;
-  if (b > (double)(n - 1)) b = (double)(n - 1);
-  if (a > b) {
+  if (l > h) {
     lo = 0;
     hi = -1;
     return;
   }
-  int l = (int)a, h = (int)b;
   while (l <= h && !in(l)) ++l;
   while (h >= l && !in(h)) --h;
   lo = l;
@@ -407,23 +414,44 @@ __device__ __forceinline__ int first_true(int n, int guess, P pred) {
   return hi;
 }
 
+// An FP64 value as an integer that orders as the value does (-0 as 0; a NaN
+// past the infinity of its sign): comparisons of these leave the few FP64
+// units alone.
+__device__ __forceinline__ long long order_key(double v) {
+  const long long b = __double_as_longlong(v);
+  const long long m = (long long)0x8000000000000000ull;
+  return b >= 0 ? b : (b == m ? 0 : m - b);
+}
+
+// A cube's channel grid for channel_range: first edge and channels per km/s,
+// for the guess that starts a search.
+struct ChanGrid {
+  float e0, scale;
+  __device__ __forceinline__ ChanGrid(const double* e, int nc, int dec) {
+    const double a = dec ? e[nc] : e[0], b = dec ? e[0] : e[nc];
+    e0 = (float)a;
+    scale = (float)nc / (float)(b - a);
+  }
+};
+
 // Channel index range whose closed velocity interval meets [lo, hi].  The
-// FP64 edge comparisons decide; a linear guess from the end edges (exact
-// for uniform channels) starts each search.
-__device__ __forceinline__ void channel_range(const double* e, int nc, int dec, double lo,
-                                              double hi, int& c0, int& c1) {
+// comparisons of the FP64 edges decide; a linear guess in FP32 from the end
+// edges starts each search (right for uniform channels but for values within
+// the FP32 rounding of an edge, which take a probe more).
+__device__ __forceinline__ void channel_range(const double* e, int nc, int dec,
+                                              const ChanGrid& grid, double lo, double hi,
+                                              float lo_f, float hi_f, int& c0, int& c1) {
   // E(k) = edges in increasing order
-  auto E = [&](int k) { return dec ? e[nc - k] : e[k]; };
-  const double e0 = E(0), en = E(nc);
-  const float scale = (float)nc / (float)(en - e0);
-  auto guess = [&](double v) {
-    const float t = floorf((float)(v - e0) * scale);
+  auto E = [&](int k) { return order_key(dec ? e[nc - k] : e[k]); };
+  auto guess = [&](float v) {
+    const float t = floorf((v - grid.e0) * grid.scale);
     return t >= 0.f ? (t < (float)nc ? (int)t : nc) : 0;  // NaN -> 0
   };
+  const long long lo_k = order_key(lo), hi_k = order_key(hi);
   // first c in [0, nc) with E(c + 1) >= lo (nc if none)
-  const int first = first_true(nc, guess(lo) - 1, [&](int c) { return E(c + 1) >= lo; });
+  const int first = first_true(nc, guess(lo_f) - 1, [&](int c) { return E(c + 1) >= lo_k; });
   // last c in [0, nc) with E(c) <= hi  ->  (first c with E(c) > hi) - 1
-  const int last = first_true(nc, guess(hi), [&](int c) { return E(c) > hi; }) - 1;
+  const int last = first_true(nc, guess(hi_f), [&](int c) { return E(c) > hi_k; }) - 1;
   if (first > last) {
     c0 = 1;
     c1 = 0;

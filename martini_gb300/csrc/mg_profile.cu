@@ -98,6 +98,7 @@ k_profile_sum(long long n, int nc, int model, const double* __restrict__ v,
   extern __shared__ double s_acc[];
   if (w.hdr->status) return;
   const int dec = *w.dec;
+  const ChanGrid grid(edges, nc, dec);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double* const acc = SMEM ? s_acc + (size_t)warp * nc : w.part + (size_t)blockIdx.x * nc;
   for (int c = lane; c < nc; c += 32) acc[c] = 0.0;
@@ -118,9 +119,11 @@ k_profile_sum(long long n, int nc, int model, const double* __restrict__ v,
         const double s = sigma ? (double)sigma[p] : (double)sigma_const;
         inv_s = (float)(1.0 / (1.4142135623730951 * s));
         const double half = 4.5 * 1.4142135623730951 * s;
-        channel_range(edges, nc, dec, vp - half, vp + half, clo, chi);
+        const float half_f = (float)half;
+        channel_range(edges, nc, dec, grid, vp - half, vp + half, vhi - half_f, vhi + half_f, clo,
+                      chi);
       } else {
-        channel_range(edges, nc, dec, vp, vp, clo, chi);
+        channel_range(edges, nc, dec, grid, vp, vp, vhi, vhi, clo, chi);
       }
       if (a == 0.0 || !isfinite(vp)) {  // mass pruning (martini.py:168-241)
         clo = 1;
