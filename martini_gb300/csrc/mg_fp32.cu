@@ -195,6 +195,31 @@ k_contract_fp32(Geo g, Ws w) {
               Ws_[q][h * 32 + lane] =
                   i + 2 * h >= ilo && i + 2 * h <= ihi ? f * scale * inv_h2 : 0.f;
             }
+          } else if (hit && kt == MG_KERNEL_GAUSSIAN) {
+            // w_gaussian's arithmetic; its row factors (lane l computes that of
+            // row l mod 8) and column factors are shared by the 128 pixels: 8
+            // error functions a lane instead of 20
+            const float trunc = s_ks[r.kslot].truncate, ign = 1.f / s_ks[r.kslot].gnorm;
+            const float inv_hs = 1.f / (r.h * 0.42466090014400953f);
+            const float sg = inv_hs * 0.70710678118654752f;
+            const float dy = (float)(r.yi - j) + r.yf;
+            const float ey = erff((dy + 0.5f) * sg) - erff((dy - 0.5f) * sg);
+            const float dxr = (float)(r.xi - (i0 + (lane & 7))) + r.xf;
+            const float exr = erff((dxr + 0.5f) * sg) - erff((dxr - 0.5f) * sg);
+            const bool in_j = r.jlo <= j && j <= r.jhi;
+#pragma unroll
+            for (int h = 0; h < TILE_I / 2; ++h) {
+              const int row = 2 * h + (lane >> 4);
+              const float ex = __shfl_sync(0xffffffffu, exr, row);
+              const float dx = (float)(r.xi - (i0 + row)) + r.xf;
+              const float dr = sqrtf(dx * dx + dy * dy);
+              const float q = dr * inv_hs;
+              const float zmax = trunc > q ? sqrtf(trunc * trunc - q * q) : 0.f;
+              const float f = 0.25f * erff(zmax * 0.70710678118654752f) * ex * ey * ign;
+              const bool in = in_j && i0 + row >= r.ilo && i0 + row <= r.ihi &&
+                              !((dr - 0.70710678118654752f) * inv_hs > trunc);
+              Ws_[warp * (F32_KC / 8) + e][h * 32 + lane] = in ? f : 0.f;
+            }
           } else {
 #pragma unroll
             for (int h = 0; h < TILE_I / 2; ++h) {
