@@ -51,7 +51,7 @@ FORMS = {"fp32": 0, "bf16x3": 1, "f16x3": 2, "bf16x6": 3}
 # DRAM bytes (read + write) of one launch of the contraction kernel, from
 # one ncu pass (dram__bytes_read.sum + dram__bytes_write.sum) on the full
 # workload, for the kernel as it stands
-TRAFFIC_BYTES = {("disc4m_1024", "bf16x6"): 5_896_006_400}
+TRAFFIC_BYTES = {("disc4m_1024", "bf16x6"): 5_181_670_400}
 
 
 def launches_per_step(form: str, lines: bool, nx: int, ny: int, nc: int, n: int, pairs: int,
