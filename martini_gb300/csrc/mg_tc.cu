@@ -651,7 +651,7 @@ __global__ void k_spec_fp32(Geo g, Ws w) {
 // Dirac lines (one channel, two for a velocity on an edge), a thread per
 // particle.  Evaluated by the producer instead, every stage read 64 records
 // from global memory in the middle of its production (200k particles, 21.5M
-// pairs: contraction 8.8 ms so, 6.6 ms with the store).
+// pairs: contraction 8.8 ms so, 6.8 ms with the store).
 __global__ void k_spec_dirac(Geo g, Ws w) {
   const bool form_fp32 = g.form == MG_FORM_BF16X6, form_bf16 = g.form == MG_FORM_BF16X3;
   const bool fits = w.hdr->n_spec <= w.cap_spec && !(w.hdr->status & ST_NO_PLAN);
