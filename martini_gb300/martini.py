@@ -32,6 +32,8 @@ def add_to_array(array, add, pads, px2, divide_all):
     more axis of length 1) in one native pass: ``(array + add) / px2`` when
     ``divide_all``, else ``array + add / px2``.  Returns the per-channel sums
     of ``array * px2`` over the pixels inside ``pads``."""
+    if array.shape not in (add.shape, (*add.shape, 1)):
+        raise ValueError(f"an inserted cube of shape {add.shape} into an array of shape {array.shape}")
     if not array.flags.writeable:
         raise ValueError("output array is read-only")
     # a view (a cube without its pad) or another type goes through a copy
