@@ -28,18 +28,29 @@ DEFAULT_FORM = "bf16x6"
 
 
 def add_to_array(array, add, pads, px2, divide_all):
-    """Add the FP32 cube ``add`` to the FP64 host ``array`` (its shape, or one
-    more axis of length 1) in one native pass: ``(array + add) / px2`` when
-    ``divide_all``, else ``array + add / px2``.  Returns the per-channel sums
-    of ``array * px2`` over the pixels inside ``pads``."""
+    """Add the FP32 cube ``add`` to the host ``array`` (its shape, or one more
+    axis of length 1), FP64 arrays in one native pass: ``(array + add) / px2``
+    when ``divide_all``, else ``array + add / px2``.  Returns the per-channel
+    sums of ``array * px2`` over the pixels inside ``pads``."""
     if array.shape not in (add.shape, (*add.shape, 1)):
         raise ValueError(f"an inserted cube of shape {add.shape} into an array of shape {array.shape}")
     if not array.flags.writeable:
         raise ValueError("output array is read-only")
-    # a view (a cube without its pad) or another type goes through a copy
-    work = np.ascontiguousarray(array, dtype=np.float64)
-    add = np.ascontiguousarray(add, dtype=np.float32)
     nx, ny, nc = add.shape
+    if array.dtype != np.float64:
+        # FP64 would not hold every type's values: the array operations, which
+        # refuse the types that hold no fractions
+        add = add.astype(np.float64).reshape(array.shape)
+        if divide_all:
+            array += add
+            array /= px2
+        else:
+            array += add / px2
+        inner = array[pads[0]:nx - pads[0], pads[1]:ny - pads[1]]
+        return (inner * px2).sum(axis=(0, 1)).reshape(-1)
+    # a view (a cube without its pad) goes through a copy
+    work = np.ascontiguousarray(array)
+    add = np.ascontiguousarray(add, dtype=np.float32)
     per_channel = np.empty(nc)
     N.check(N.load().mg_cube_add(work.ctypes.data, add.ctypes.data, nx, ny, nc, *pads, float(px2),
                                  int(divide_all), per_channel.ctypes.data))

@@ -18,3 +18,34 @@ def test_another_shape_is_refused(shape, add, divide_all):
     with pytest.raises(ValueError, match="shape"):
         add_to_array(arr, np.ones(add, np.float32), (0, 0), 2.0, divide_all)
     assert np.all(arr == 1.0)
+
+
+@pytest.mark.parametrize("divide_all", [True, False])
+@pytest.mark.parametrize("dtype", ["f4", ">f8", "c16", "g"])
+def test_other_types_as_the_array_operations(dtype, divide_all):
+    rng = np.random.default_rng(1)
+    add = rng.uniform(0, 1, (6, 7, 5)).astype(np.float32)
+    arr = rng.uniform(0, 1, (6, 7, 5, 1)).astype(dtype)
+    if dtype == "c16":
+        arr += 1j
+    if dtype == "g":
+        arr += np.longdouble(2) ** -60  # lost in FP64
+    want = arr.copy()
+    if divide_all:
+        want += add.astype(np.float64)[..., np.newaxis]
+        want /= 3.7
+    else:
+        want += add.astype(np.float64)[..., np.newaxis] / 3.7
+    got = add_to_array(arr, add, (1, 2), 3.7, divide_all)
+    assert arr.dtype == np.dtype(dtype) and np.array_equal(arr, want)
+    inner = (want[1:-1, 2:-2] * 3.7).sum(axis=(0, 1)).reshape(-1)
+    assert np.array_equal(got, inner)
+
+
+@pytest.mark.parametrize("divide_all", [True, False])
+@pytest.mark.parametrize("dtype", [np.int64, np.uint8, bool])
+def test_types_that_hold_no_fractions_are_refused(dtype, divide_all):
+    arr = np.ones((4, 5, 3), dtype)
+    with pytest.raises(TypeError):
+        add_to_array(arr, np.full((4, 5, 3), 0.5, np.float32), (0, 0), 2.0, divide_all)
+    assert np.all(arr == 1)
