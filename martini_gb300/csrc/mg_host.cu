@@ -12,7 +12,6 @@
 #include <atomic>
 #include <exception>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -75,8 +74,9 @@ extern "C" int mg_cube_add(double* array, const float* add, int64_t nx, int64_t 
     pool.reserve(HOST_THREADS);
     try {
       for (long long t = 1; t < want; ++t) pool.emplace_back(work);
-    } catch (const std::system_error&) {
-      // no more threads to be had: the ones there and this one do the work
+    } catch (const std::exception&) {
+      // no more threads (or memory for one) to be had: the ones there and this
+      // one do the work; they must be joined before the pool goes
     }
     work();
     for (std::thread& t : pool) t.join();
