@@ -427,7 +427,10 @@ __global__ void k_resume(Geo g, Ws w, int num_sms, long long cap_pairs, long lon
   WsHeader* h = w.hdr;
   const bool ok = h->plan_key == plan_key;
   const long long total = ok ? h->n_pairs : 0;
-  h->status = ok ? (total > cap_pairs ? ST_PAIRS : 0u) : (ST_NO_PLAN | ST_PAIRS);
+  // bad channel edges stay an error of the run, as they were of the plan; the
+  // plan's pair status does not (it ran without room for pairs)
+  h->status = ok ? (h->status & ST_EDGES) | (total > cap_pairs ? ST_PAIRS : 0u)
+                 : (ST_NO_PLAN | ST_PAIRS);
   h->item_counter = 0;
   h->reduce_counter = 0;
   h->n_pairs = total;
