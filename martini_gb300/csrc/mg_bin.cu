@@ -80,10 +80,13 @@ void launch_set_gals(const Gal* gals, const Geo& g, const Ws& w, cudaStream_t s)
 // 5.7 ms), 20 % on 500k wide ones in 1024^2 x 256 (30.4 to 25.8 ms).  `reach2`
 // is the squared radius in px with a margin far above the rounding of the FP32
 // weights (2e-5 relative and 2e-4 px); a kernel without a radius (Dirac: its box
-// is one pixel) or with one past 1e8 px keeps the whole box.  Rounded operations
-// only, so that the counts and the list agree whatever the compiler fuses.
+// is one pixel) or with one past 1e8 px keeps the whole box.  So does a particle
+// whose line or weights may not be finite: zero weights make NaN of an infinite
+// line, and a length of zero makes NaN of every weight, all over the box.
+// Rounded operations only, so that the counts and the list agree whatever the
+// compiler fuses.
 __device__ __forceinline__ float reach2(const PRec& r, const KSpec& k) {
-  if (k.type == MG_KERNEL_DIRAC) return 1e30f;
+  if (k.type == MG_KERNEL_DIRAC || !(fabsf(r.amp) < 1e30f) || !(r.inv_h2 < 1e30f)) return 1e30f;
   const float rad = k.type == MG_KERNEL_GAUSSIAN
                         ? __fmul_rn(k.truncate, __fmul_rn(r.h, 0.42466090014400953f))
                         : r.h;
@@ -111,6 +114,25 @@ __device__ __forceinline__ void row_tiles(int xi, float xf, int yi, float yf, in
   }
   t0 = jlo / TILE_J;
   t1 = jhi / TILE_J;
+}
+
+// Whether a particle's tabulated spectrum holds a value that reach2 takes for
+// not finite, into the pair counts (which the records kernel reads and
+// overwrites); a warp per particle.  One more pass over the table, bound by
+// HBM: 57 us for 500k spectra of 128 channels (bf16x6 insertion 1.34 to 1.40
+// ms; 1.60 ms with the whole box of every particle listed).
+__global__ void k_table_finite(Geo g, Ws w) {
+  const int lane = threadIdx.x & 31;
+  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long P = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; P < g.n;
+       P += nwarps) {
+    const Gal& G = w.gal[find_gal(w.gp0, g.ngal, P)];
+    const float* s = G.spectra + (P - G.p0) * G.nc;
+    bool bad = false;
+    for (int c = lane; c < G.nc; c += 32) bad |= !(fabsf(s[c]) < 1e30f);
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) w.npairs[P] = bad;
+  }
 }
 
 constexpr int PREP_THREADS = 256;
@@ -202,7 +224,7 @@ __global__ void __launch_bounds__(PREP_THREADS) k_prep(Geo g, Ws w, long long pe
         if (g.spectral_model == MG_SPECTRUM_TABLE) {
           rec.clo = 0;
           rec.chi = G.nc - 1;
-          rec.amp = 1.f;
+          rec.amp = w.npairs[P] ? __int_as_float(0x7f800000) : 1.f;  // k_table_finite
         } else {
           double v = G.v[p];
           double am = G.amp[p];
@@ -668,6 +690,8 @@ void launch_prep(const Geo& g, const Ws& w, int num_sms, cudaStream_t s, long lo
   k_tile_init<<<grid_for(init_n, num_sms), 256, 0, s>>>(g, w, cap_pairs, cap_partial);
   k_edges<<<grid_for(g.nedge, num_sms), 256, 0, s>>>(g, w);
   if (g.n > 0) {
+    if (g.spectral_model == MG_SPECTRUM_TABLE)
+      k_table_finite<<<grid_for(g.n * 32, num_sms), 256, 0, s>>>(g, w);
     // every block adds its arrays to the global ones: fewer, longer runs where
     // the arrays are large
     const int nd = g.max_diff <= PREP_SMEM_DIFF ? g.max_diff : g.ngal > 1 ? PREP_SMEM_DIFF : 0;
