@@ -282,8 +282,8 @@ int radix_passes(int bits);
 void launch_radix_sort(unsigned* keys, int* vals, unsigned* kt, int* vt, const long long* np,
                        long long cap, int bits, int* hist, long long* off, long long* sums,
                        cudaStream_t s);
-void launch_order_particles(const Geo& g, const Ws& w, int* out, long long max_chunks, int* hist,
-                            long long* off, cudaStream_t s);
+void launch_order_particles(const Geo& g, const Ws& w, int* out, int* hist, long long* off,
+                            cudaStream_t s);
 int launch_contract_fp32(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
 int launch_contract_bf16x3(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);
 void launch_reduce_partials(const Geo& g, const Ws& w, int num_sms, cudaStream_t s);

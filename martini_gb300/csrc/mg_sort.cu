@@ -403,9 +403,12 @@ void launch_radix_sort(unsigned* keys, int* vals, unsigned* kt, int* vt, const l
 }
 
 // The particles with pairs in order of kernel class and first channel:
-// their indices into `out`, their number into hdr->n_valid.
-void launch_order_particles(const Geo& g, const Ws& w, int* out, long long max_chunks, int* hist,
-                            long long* off, cudaStream_t s) {
+// their indices into `out`, their number into hdr->n_valid.  hist and off
+// need 2^RS_BITS * radix_chunks(g.n) entries where there are several chunks
+// (g.n > 2 RS_TILE, so that scan_sums, which has room for g.n, has room for
+// those too).
+void launch_order_particles(const Geo& g, const Ws& w, int* out, int* hist, long long* off,
+                            cudaStream_t s) {
   RsParticles el{w.rec, w.npairs, w.hdr, out, g.n, 0, {}};
   while (((g.max_nc - 1) >> el.cshift) > 127) ++el.cshift;
   for (int k = 0; k < g.n_kernels; ++k) {
@@ -414,9 +417,7 @@ void launch_order_particles(const Geo& g, const Ws& w, int* out, long long max_c
                 : t == MG_KERNEL_DIRAC                                     ? 1
                                                                             : 0;
   }
-  long long chunks = radix_chunks(g.n);
-  if (chunks > max_chunks) chunks = max_chunks;
-  rs_pass(el, RS_BITS, chunks, hist, off, w.scan_sums, &w.hdr->n_valid, s);
+  rs_pass(el, RS_BITS, radix_chunks(g.n), hist, off, w.scan_sums, &w.hdr->n_valid, s);
 }
 
 }  // namespace mg
