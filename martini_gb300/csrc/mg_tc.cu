@@ -626,25 +626,41 @@ __global__ void k_spec_eval(Geo g, Ws w) {
   }
 }
 
-// The FP32 form's lines, by its own line function (the same bits as lines
-// evaluated in the contraction), a warp per particle.
-__global__ void k_spec_fp32(Geo g, Ws w) {
+// The FP32 form's Gaussian lines, by its own line function (the same bits as
+// lines evaluated in the contraction).  Short lines are bound by the latency of
+// a particle's record and offset, so a warp takes four particles at once, eight
+// lanes each: 500k lines of 25 channels 193 us with a warp per particle (more
+// than the contraction gained where each particle meets one tile), 133 us now.
+// Long lines are bound by the error functions, whose branches a warp's lanes
+// share best on one line: with one past 32 channels, the four in turn.
+// `quad`: 4, or 1 where there are warps enough for a particle each.
+__global__ void k_spec_fp32(Geo g, Ws w, int quad) {
   const bool fits = w.hdr->n_spec <= w.cap_spec && !(w.hdr->status & ST_NO_PLAN);
   if (blockIdx.x == 0 && threadIdx.x == 0) w.hdr->spec_ready = fits ? 1 : 0;
   if (!fits) return;
   const int lane = threadIdx.x & 31;
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long p = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; p < g.n;
-       p += nwarps) {
-    const int cnt = w.npairs[p];
-    if (cnt <= 0) continue;
+  auto line = [&](long long p, int cnt, int first, int step) {
     const PRec r = w.rec[p];
     const int gk = find_gal(w.gp0, g.ngal, p);
     const int e0 = w.gal[gk].edge0, dec = w.gst[gk].dec;
     unsigned* out = w.spec + w.pair_off[p];
-    for (int m = lane; m < cnt; m += 32)
+    for (int m = first; m < cnt; m += step)
       out[m] = __float_as_uint(channel_spectrum(r, g.spectral_model, r.clo + m, dec, w.ehi + e0,
                                                 w.elo + e0, w.inv_w + e0));
+  };
+  for (long long base = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * quad;
+       base < g.n; base += nwarps * quad) {
+    const long long p = base + (lane >> 3);
+    const int cnt = (lane >> 3) < quad && p < g.n ? w.npairs[p] : 0;
+    if (quad == 1 || __any_sync(0xffffffffu, cnt > 32)) {
+      for (int k = 0; k < quad; ++k) {
+        const int ck = __shfl_sync(0xffffffffu, cnt, 8 * k);
+        if (ck > 0) line(base + k, ck, lane, 32);
+      }
+    } else if (cnt > 0) {
+      line(p, cnt, lane & 7, 8);
+    }
   }
 }
 
@@ -653,7 +669,8 @@ __global__ void k_spec_fp32(Geo g, Ws w) {
 // from global memory in the middle of its production (200k particles, 21.5M
 // pairs: contraction 8.8 ms so, 6.8 ms with the store).
 __global__ void k_spec_dirac(Geo g, Ws w) {
-  const bool form_fp32 = g.form == MG_FORM_BF16X6, form_bf16 = g.form == MG_FORM_BF16X3;
+  const bool form_fp32 = g.form == MG_FORM_BF16X6 || g.form == MG_FORM_FP32;
+  const bool form_bf16 = g.form == MG_FORM_BF16X3;
   const bool fits = w.hdr->n_spec <= w.cap_spec && !(w.hdr->status & ST_NO_PLAN);
   if (blockIdx.x == 0 && threadIdx.x == 0) w.hdr->spec_ready = fits ? 1 : 0;
   if (!fits) return;
@@ -1764,13 +1781,15 @@ void launch_spec_store(const Geo& g, const Ws& w, int num_sms, cudaStream_t s) {
   const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, (long long)num_sms * 16);
   k_spec_count<<<blocks, 256, 0, s>>>(g, w);
   launch_scan(w.npairs, n, w.pair_off, w.scan_sums, &w.hdr->n_spec, s);
-  if (g.form == MG_FORM_FP32) {
-    k_spec_fp32<<<(unsigned)std::min<long long>((n + 7) / 8, (long long)num_sms * 32), 256, 0, s>>>(
-        g, w);
-    return;
-  }
   if (g.spectral_model == MG_SPECTRUM_DIRAC) {
     k_spec_dirac<<<blocks, 256, 0, s>>>(g, w);
+    return;
+  }
+  if (g.form == MG_FORM_FP32) {
+    const int quad = n > (long long)num_sms * 64 ? 4 : 1;
+    const long long warps = (n + quad - 1) / quad;
+    k_spec_fp32<<<(unsigned)std::min<long long>((warps + 7) / 8, (long long)num_sms * 32), 256, 0,
+                  s>>>(g, w, quad);
     return;
   }
   // a warp per particle, many warps in flight (each particle's work is a
