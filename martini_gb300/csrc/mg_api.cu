@@ -521,7 +521,8 @@ int run(const mg_problem* probs, int nprob, void* ws, size_t bytes, cudaStream_t
         k_clear_cubes<<<dim3(64, (unsigned)g.ngal), 256, 0, s>>>(g, w);
       }
     }
-    if (e == cudaSuccess) e = cudaMemsetAsync(&w.hdr->item_counter, 0, sizeof(unsigned), s);
+    if (e == cudaSuccess)
+      e = cudaMemsetAsync(&w.hdr->item_counter, 0, sizeof(unsigned) + sizeof(w.hdr->sm_blocks), s);
     if (e != cudaSuccess) return cuda_fail(e, "cube clear");
     if (tc_form(g.form)) {
       rc = launch_contract_bf16x3(g, w, num_sms(), s);

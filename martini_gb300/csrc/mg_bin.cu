@@ -332,7 +332,6 @@ __global__ void k_tile_init(Geo g, Ws w, long long cap_pairs, long long cap_part
     WsHeader* h = w.hdr;
     h->status = 0;
     h->item_counter = 0;
-    h->reduce_counter = 0;
     h->n_pairs = h->n_items = h->n_partial_items = h->partial_bound = 0;
     h->cap_pairs = cap_pairs;
     h->cap_partial_items = cap_partial;
@@ -454,7 +453,6 @@ __global__ void k_resume(Geo g, Ws w, int num_sms, long long cap_pairs, long lon
   h->status = ok ? (h->status & ST_EDGES) | (total > cap_pairs ? ST_PAIRS : 0u)
                  : (ST_NO_PLAN | ST_PAIRS);
   h->item_counter = 0;
-  h->reduce_counter = 0;
   h->n_pairs = total;
   h->n_items = h->n_partial_items = 0;
   h->n_valid = 0;

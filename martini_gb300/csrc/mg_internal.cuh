@@ -178,12 +178,14 @@ constexpr unsigned ST_EDGES = 4u;        // channel edges not strictly monotonic
 constexpr unsigned ST_TIMEOUT = 8u;      // a bounded device-side wait expired
 constexpr unsigned ST_NO_PLAN = 16u;     // no plan of the problem to continue from
 
+constexpr int SM_BUCKETS = 152;  // SMs of this part, 4 a word
+
 // Workspace header (device): status flags and scalar counters.
 struct WsHeader {
   unsigned int status;           // ST_* bits
   unsigned int item_counter;     // dynamic scheduler cursor
-  unsigned int reduce_counter;
-  int pad0;
+  unsigned int sm_blocks[SM_BUCKETS / 4];  // blocks of the FP32 contraction started on each
+                                           // SM, a byte each; cleared with the cursor
   long long n_pairs;
   long long n_items;
   long long n_partial_items;
@@ -197,6 +199,7 @@ struct WsHeader {
   long long n_valid;             // particles with pairs (particle list stage)
   unsigned long long plan_key;   // problem whose plan the workspace holds, 0: none
 };
+static_assert(sizeof(WsHeader) <= 256, "header slot of the workspace");
 
 // Pointers into the workspace (host computes, passes by value).  Arrays run
 // over the whole batch.  A "segment" is one (tile, channel block) of the
