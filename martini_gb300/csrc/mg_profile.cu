@@ -14,6 +14,13 @@
 // Bound by the error functions, one per (particle, support edge): before, a
 // thread per channel walked every particle of its block, and 1,000,000
 // particles on 256 channels took 1.01 ms; now 0.38 ms (a call).
+// A warp's lines are one chain, so where there are few particles they are dealt
+// to more blocks and all warps, and the band to blocks of channels (which also
+// keeps eight warps' spectra in shared memory whatever the band).  With whole
+// bands and 1024 particles a block, 400 lines across 8192 channels took 15.5 ms a
+// call and 32 across 256 143 us (1.9 ms and 81 us with a thread per channel);
+// 130 and 67 us now, 20k lines of 28 channels 118 and 74 us.
+#include <algorithm>
 #include <string>
 
 #include "mg_internal.cuh"
@@ -27,9 +34,12 @@ namespace {
 using namespace mg;
 
 constexpr int PROF_WARPS = 8;          // warps per block
-constexpr int PROF_PER_BLOCK = 1024;   // particles per block, while the blocks suffice
+constexpr int PROF_PER_BLOCK = 1024;   // most particles per block, while the blocks suffice
 constexpr int PROF_MAX_BLOCKS = 2048;
-constexpr size_t PROF_SMEM = 96 * 1024;  // the warps' spectra
+constexpr int PROF_FILL = 152;         // blocks that fill the chip's SMs
+constexpr long long PROF_PART = 1 << 22;  // partial sums (32 MB) that more blocks may take
+constexpr int PROF_CHUNK = 1536;       // most channels per block: 96 KB of the warps' spectra
+constexpr int PROF_MIN_CHUNK = 64;
 constexpr int PROF_CH = 32, PROF_GROUPS = 16;  // channels, block groups of k_profile_final
 
 struct ProfWs {
@@ -43,10 +53,23 @@ struct ProfWs {
 
 size_t al(size_t x) { return (x + 255) & ~size_t(255); }
 
-int prof_blocks(long long n) {
-  long long b = (n + PROF_PER_BLOCK - 1) / PROF_PER_BLOCK;
-  if (b > PROF_MAX_BLOCKS) b = PROF_MAX_BLOCKS;
+// Particle ranges, a block (or one per channel chunk) each: PROF_PER_BLOCK
+// particles, fewer while that leaves SMs idle, but one for each warp.
+int prof_blocks(long long n, int nc) {
+  const long long full = (n + PROF_PER_BLOCK - 1) / PROF_PER_BLOCK;
+  long long b = std::min<long long>((n + PROF_WARPS - 1) / PROF_WARPS, 2 * PROF_FILL);
+  b = std::max(std::min(b, PROF_PART / nc), full);
+  b = std::min<long long>(b, PROF_MAX_BLOCKS);
   return (int)(b > 0 ? b : 1);
+}
+
+// Channels of a block's chunk: the band in equal chunks of at most PROF_CHUNK,
+// smaller while the blocks do not fill the chip.
+int prof_chunk(int nc, int blocks) {
+  long long k = (nc + PROF_CHUNK - 1) / PROF_CHUNK;
+  const long long fill = (PROF_FILL + blocks - 1) / blocks;
+  k = std::max<long long>(k, std::min<long long>(fill, (nc + PROF_MIN_CHUNK - 1) / PROF_MIN_CHUNK));
+  return (int)(((nc + k - 1) / k + 31) / 32 * 32);
 }
 
 size_t prof_layout(long long n, int nc, size_t* off) {
@@ -56,7 +79,7 @@ size_t prof_layout(long long n, int nc, size_t* off) {
   off[2] = o; o += al(sizeof(float) * (size_t)(nc + 1));
   off[3] = o; o += al(sizeof(float) * (size_t)(nc + 1));
   off[4] = o; o += al(sizeof(int));
-  off[5] = o; o += al(sizeof(double) * (size_t)prof_blocks(n) * nc);
+  off[5] = o; o += al(sizeof(double) * (size_t)prof_blocks(n, nc) * nc);
   return o;
 }
 
@@ -88,28 +111,30 @@ __device__ __forceinline__ float profile_edge(float vhi, float vlo, float inv_s,
   return erfcf(fabsf(u));
 }
 
-// SMEM: the warps' spectra in shared memory; else (bands too wide for it) one
-// warp per block adds to the block's row of the partial sums.
-template <bool SMEM>
+// Block (x, y): particle range x, channels [y chunk, (y + 1) chunk).
 __global__ void __launch_bounds__(PROF_WARPS * 32)
-k_profile_sum(long long n, int nc, int model, const double* __restrict__ v,
+k_profile_sum(long long n, int nc, int chunk, int model, const double* __restrict__ v,
               const float* __restrict__ sigma, float sigma_const,
               const double* __restrict__ amp, const double* __restrict__ edges, ProfWs w) {
-  extern __shared__ double s_acc[];
+  extern __shared__ double s_acc[];  // [warp][chunk]
   if (w.hdr->status) return;
   const int dec = *w.dec;
   const ChanGrid grid(edges, nc, dec);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  double* const acc = SMEM ? s_acc + (size_t)warp * nc : w.part + (size_t)blockIdx.x * nc;
-  for (int c = lane; c < nc; c += 32) acc[c] = 0.0;
+  const int c0 = blockIdx.y * chunk, c1 = min(c0 + chunk, nc);
+  double* const acc = s_acc + (size_t)warp * chunk - c0;  // this warp's, by channel
+  for (int c = c0 + lane; c < c1; c += 32) acc[c] = 0.0;
   const long long per = (n + gridDim.x - 1) / gridDim.x;
   const long long p1 = min((long long)(blockIdx.x + 1) * per, n);
-  // a lane only ever touches its own channels: no barrier between particles
-  for (long long p0 = (long long)blockIdx.x * per + warp * 32; p0 < p1; p0 += 32 * nw) {
+  // particles a warp takes at a time: all warps' shares where the range is short
+  const int at = (int)min(32ll, (per + nw - 1) / nw);
+  // a lane only ever touches its own channels (c0 is a multiple of 32): no
+  // barrier between particles
+  for (long long p0 = (long long)blockIdx.x * per + warp * at; p0 < p1; p0 += at * nw) {
     const long long p = p0 + lane;
     float vhi = 0.f, vlo = 0.f, inv_s = 0.f, am = 0.f;
     int clo = 1, chi = 0;
-    if (p < p1) {
+    if (lane < at && p < p1) {
       const double vp = v[p], a = amp[p];
       const double vh = (double)(float)vp;
       vhi = (float)vh;
@@ -129,8 +154,10 @@ k_profile_sum(long long n, int nc, int model, const double* __restrict__ v,
         clo = 1;
         chi = 0;
       }
+      clo = max(clo, c0);
+      chi = min(chi, c1 - 1);
     }
-    const int m = (int)min(32ll, p1 - p0);
+    const int m = (int)min((long long)at, p1 - p0);
     for (int k = 0; k < m; ++k) {
       const int a = __shfl_sync(0xffffffffu, clo, k), b = __shfl_sync(0xffffffffu, chi, k);
       if (a > b) continue;
@@ -162,11 +189,10 @@ k_profile_sum(long long n, int nc, int model, const double* __restrict__ v,
       }
     }
   }
-  if (!SMEM) return;
   __syncthreads();
-  for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+  for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
     double t = 0.0;
-    for (int k = 0; k < nw; ++k) t += s_acc[(size_t)k * nc + c];
+    for (int k = 0; k < nw; ++k) t += s_acc[(size_t)k * chunk + (c - c0)];
     w.part[(size_t)blockIdx.x * nc + c] = t;
   }
 }
@@ -237,26 +263,19 @@ extern "C" int mg_global_profile(const mg_problem* p, double* spectrum, void* wo
   }
   // one block, so the edge direction is known before the range checks
   k_profile_edges<<<1, 256, 0, s>>>(p->edges, p->nc, w);
-  const int nb = prof_blocks(p->n);
+  const int nb = prof_blocks(p->n, p->nc);
   if (p->n > 0) {
-    // as many warps per block as their spectra fit in shared memory
-    const size_t row = sizeof(double) * (size_t)p->nc;
-    int warps = (int)(PROF_SMEM / row);
-    if (warps > PROF_WARPS) warps = PROF_WARPS;
-    if (warps > 0) {
-      if (warps * row > 48 * 1024 &&
-          cudaFuncSetAttribute(k_profile_sum<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)PROF_SMEM) != cudaSuccess) {
-        mg::set_last_error("mg_global_profile: shared memory attribute");
-        return MG_ERR_CUDA;
-      }
-      k_profile_sum<true><<<nb, warps * 32, warps * row, s>>>(p->n, p->nc, p->spectral_model, p->v,
-                                                              p->sigma, p->sigma_const, p->amp,
-                                                              p->edges, w);
-    } else {
-      k_profile_sum<false><<<nb, 32, 0, s>>>(p->n, p->nc, p->spectral_model, p->v, p->sigma,
-                                             p->sigma_const, p->amp, p->edges, w);
+    const int chunk = prof_chunk(p->nc, nb);
+    const size_t smem = sizeof(double) * (size_t)PROF_WARPS * chunk;
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(k_profile_sum, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(sizeof(double) * PROF_WARPS * PROF_CHUNK)) != cudaSuccess) {
+      mg::set_last_error("mg_global_profile: shared memory attribute");
+      return MG_ERR_CUDA;
     }
+    k_profile_sum<<<dim3((unsigned)nb, (unsigned)((p->nc + chunk - 1) / chunk)), PROF_WARPS * 32,
+                    smem, s>>>(p->n, p->nc, chunk, p->spectral_model, p->v, p->sigma,
+                               p->sigma_const, p->amp, p->edges, w);
   } else {
     cudaMemsetAsync(w.part, 0, sizeof(double) * (size_t)nb * p->nc, s);
   }
