@@ -113,9 +113,15 @@ class InsertionEngine:
         N.check(self.lib.mg_plan(C.byref(prob), C.c_void_p(ws.data_ptr()), ws.numel(),
                                  C.c_void_p(s.cuda_stream), C.byref(info)))
         self._caps = (int(info.n_pairs), int(info.n_partial_items))
-        # the plan's size includes the spectrum store of the tensor-core forms;
-        # a workspace that had to grow no longer holds the binning
-        self._binned = self._workspace(int(info.workspace_bytes)) is ws
+        # the plan's size includes the spectrum store; a workspace that had to
+        # grow no longer holds the binning
+        try:
+            grown = self._workspace(int(info.workspace_bytes))
+        except torch.cuda.OutOfMemoryError:
+            # no room for the store: lines evaluated in the contraction
+            N.check(self.lib.mg_workspace_size(C.byref(prob), *self._caps, C.byref(base)))
+            grown = self._workspace(base.value)
+        self._binned = grown is ws
         self.last_plan = info
         return info
 
@@ -252,7 +258,12 @@ class BatchInsertion:
         N.check(self.lib.mg_plan_batched(self.arr, self.n, C.c_void_p(ws.data_ptr()), ws.numel(),
                                          self._stream(stream), C.byref(info)))
         self._caps = (int(info.n_pairs), int(info.n_partial_items))
-        self._workspace(int(info.workspace_bytes))
+        try:
+            self._workspace(int(info.workspace_bytes))
+        except torch.cuda.OutOfMemoryError:  # as in InsertionEngine.plan
+            N.check(self.lib.mg_workspace_size_batched(self.arr, self.n, *self._caps,
+                                                       C.byref(base)))
+            self._workspace(base.value)
         self.last_plan = info
         return info
 
