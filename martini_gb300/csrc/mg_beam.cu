@@ -16,7 +16,7 @@
 // memory once for many of them: a lane loads a window of 16 + T - 1 pixels and
 // applies T = 8 taps of two kernel rows to it, 128 paired FMAs for 23 loads (one
 // load per FMA before: 9.70 ms on 512 x 512 x 256 with a 27 px beam; now
-// 2.29 ms, 1.23 ms of it at the FP32 FMA rate).  Input rows stream through a ring in shared memory (cp.async,
+// 2.16 ms, 1.23 ms of it at the FP32 FMA rate).  Input rows stream through a ring in shared memory (cp.async,
 // BR_AHEAD rows ahead): at step s warp w takes input row 2 w + s, so that every
 // warp works on kernel rows kx - 1 - s and kx - s and only 15 rows are live.
 // That leaves room for two blocks on an SM, and the ring's size depends on ky
@@ -142,19 +142,24 @@ k_beam_conv(const float* __restrict__ in, int nx, int ny, int nc, int px, int py
   const int rb = i0 - (kx - 1) / 2, cb = j0 - (ky - 1) / 2;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int nrows = BT_I + kx - 1;
+  // a thread copies the same channels of every QS-th pixel of a row: what does
+  // not depend on the row is taken out of the copy, whose instructions bound
+  // small beams (3 px on 48 x 48 x 33, copied a channel at a time: 12.6 us, 8.9 now;
+  // 10.9 us with the whole halo staged before the sums)
+  constexpr int V = VEC ? 4 : 1, LPP = BC / V, QS = BEAM_THREADS / LPP;
+  const int q0 = tid / LPP, cc = (tid % LPP) * V;
+  const int qlo = c0 + cc < nc ? max(-cb, 0) : hj, qhi = min(hj, ny - cb);  // pixels in the cube
+  const long long qoff = (long long)(cb + q0) * nc + c0 + cc, qstep = (long long)QS * nc;
+  const unsigned dst0 = (unsigned)__cvta_generic_to_shared(ring + q0 * BC + cc);
   auto load_row = [&](int r) {  // input row r of the block into its ring slot
     if (r < nrows) {
       const int gi = rb + r;
       const bool row_in = gi >= 0 && gi < nx;
-      const float* const src = in + (long long)(row_in ? gi : 0) * ny * nc;
-      float* const dst = ring + (size_t)(r % BR_RING) * hj * BC;
-      constexpr int V = VEC ? 4 : 1;
-      for (int e = tid; e < hj * (BC / V); e += BEAM_THREADS) {
-        const int q = e / (BC / V), c = (e - q * (BC / V)) * V;
-        const int gj = cb + q;
-        const bool ok = row_in && gj >= 0 && gj < ny && c0 + c < nc;
-        const float* g = ok ? src + (long long)gj * nc + c0 + c : in;
-        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + q * BC + c);
+      const float* src = in + (long long)gi * ny * nc + qoff;
+      unsigned d = dst0 + (unsigned)(r % BR_RING) * (unsigned)(hj * BC * 4);
+      for (int q = q0; q < hj; q += QS, src += qstep, d += QS * BC * 4) {
+        const bool ok = row_in && q >= qlo && q < qhi;
+        const float* const g = ok ? src : in;
         if (VEC)
           asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(g),
                        "r"(ok ? 16 : 0)
