@@ -48,9 +48,9 @@ def add_to_array(array, add, pads, px2, divide_all):
             array += add / px2
         inner = array[pads[0]:nx - pads[0], pads[1]:ny - pads[1]]
         return (inner * px2).sum(axis=(0, 1)).reshape(-1)
-    # a view (a cube without its pad) goes through a copy
-    work = np.ascontiguousarray(array)
-    add = np.ascontiguousarray(add, dtype=np.float32)
+    # a view (a cube without its pad) or one off its alignment goes through a copy
+    work = np.require(array, requirements=("C", "A"))
+    add = np.require(add, np.float32, ("C", "A"))
     per_channel = np.empty(nc)
     N.check(N.load().mg_cube_add(work.ctypes.data, add.ctypes.data, nx, ny, nc, *pads, float(px2),
                                  int(divide_all), per_channel.ctypes.data))

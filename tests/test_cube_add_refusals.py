@@ -49,3 +49,24 @@ def test_types_that_hold_no_fractions_are_refused(dtype, divide_all):
     with pytest.raises(TypeError):
         add_to_array(arr, np.full((4, 5, 3), 0.5, np.float32), (0, 0), 2.0, divide_all)
     assert np.all(arr == 1)
+
+
+def test_the_native_pass_gets_aligned_arrays(monkeypatch):
+    from martini_gb300 import martini as m
+    lib = m.N.load()
+    seen = []
+
+    class Lib:
+        @staticmethod
+        def mg_cube_add(array, add, *rest):
+            seen.append((array % 8, add % 4))
+            return lib.mg_cube_add(array, add, *rest)
+
+    monkeypatch.setattr(m.N, "load", lambda: Lib)
+    shape, n = (3, 4, 5), 60
+    arr = np.frombuffer(bytearray(n * 8 + 4), dtype=np.float64, offset=4, count=n).reshape(shape)
+    add = np.frombuffer(bytearray(n * 4 + 1), dtype=np.float32, offset=1, count=n).reshape(shape)
+    add[...] = 0.5
+    assert not arr.flags.aligned and not add.flags.aligned
+    add_to_array(arr, add, (0, 0), 2.0, True)
+    assert seen == [(0, 0)] and np.all(arr == 0.25)
