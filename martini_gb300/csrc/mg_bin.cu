@@ -138,6 +138,15 @@ __global__ void k_table_finite(Geo g, Ws w) {
 constexpr int PREP_THREADS = 256;
 constexpr int PREP_SMEM_DIFF = 11776;  // 46 KB: static and dynamic within 48 KB
 
+// RUNS: a block takes its run cube by cube, as above.  Batches of cubes with few
+// particles (at most PREP_FEW on average) are taken without: a cube's turn costs a
+// block about 4 us whatever its particles, and a run has many such cubes, while
+// few particles meet on a counter.  Binning of 3000 cubes with one particle each:
+// 3.08 ms with runs, 1.83 now (1.7 ms of both sets the cubes' table up); 1000 cubes
+// of 32^3 with 64 particles each 782 us without runs, with 65 each 802 us with.
+constexpr long long PREP_FEW = 64;
+
+template <bool RUNS>
 __global__ void __launch_bounds__(PREP_THREADS) k_prep(Geo g, Ws w, long long per) {
   extern __shared__ int s_diff[];  // the difference array of the cube when it fits
   __shared__ unsigned long long s_spec;
@@ -147,20 +156,22 @@ __global__ void __launch_bounds__(PREP_THREADS) k_prep(Geo g, Ws w, long long pe
   const long long run1 = min((long long)(blockIdx.x + 1) * per, g.n);
   for (long long run0 = (long long)blockIdx.x * per; run0 < run1;) {
     // the run's particles of one cube
-    const int gk = find_gal(w.gp0, g.ngal, run0);
-    const Gal& G = w.gal[gk];
-    const long long run_hi = min(run1, w.gp0[gk + 1]);
-    const int nd = (G.ntx + 1) * (G.nty + 1);
-    const bool smem_hist = nd <= PREP_SMEM_DIFF;
+    const int run_gk = find_gal(w.gp0, g.ngal, run0);
+    const long long run_hi = RUNS ? min(run1, w.gp0[run_gk + 1]) : run1;
+    const int nd = (w.gal[run_gk].ntx + 1) * (w.gal[run_gk].nty + 1);
+    const bool smem_hist = RUNS && nd <= PREP_SMEM_DIFF;
     if (smem_hist)
       for (int t = threadIdx.x; t < nd; t += blockDim.x) s_diff[t] = 0;
     __syncthreads();
     int wmax_v = 0;
     unsigned wb_v = 0u, sb_v = 0u;
-    const ChanGrid grid(G.edges, G.nc, w.gst[gk].dec);
+    const ChanGrid run_grid(w.gal[run_gk].edges, w.gal[run_gk].nc, w.gst[run_gk].dec);
     for (long long P = run0 + threadIdx.x; P < run_hi; P += PREP_THREADS) {
+      const int gk = RUNS ? run_gk : find_gal(w.gp0, g.ngal, P);
+      const Gal& G = w.gal[gk];
       const long long p = P - G.p0;
       const int dec = w.gst[gk].dec;
+      const ChanGrid grid = RUNS ? run_grid : ChanGrid(G.edges, G.nc, dec);
       const double* edges = G.edges;
       PRec rec;
       rec.ilo = 0; rec.ihi = -1; rec.jlo = 0; rec.jhi = -1;
@@ -291,7 +302,16 @@ __global__ void __launch_bounds__(PREP_THREADS) k_prep(Geo g, Ws w, long long pe
         }
       }
       w.npairs[P] = np;
+      if (!RUNS) {
+        if (wmax_v) atomicMax(&w.gst[gk].wmax, wmax_v);
+        if (wb_v) atomicMax(&w.gst[gk].wbound_bits, wb_v);
+        if (sb_v) atomicMax(&w.gst[gk].sbound_bits, sb_v);
+        wmax_v = 0;
+        wb_v = sb_v = 0u;
+      }
     }
+    if (!RUNS) break;
+    const int gk = run_gk;
     wmax_v = __reduce_max_sync(0xffffffffu, wmax_v);
     wb_v = __reduce_max_sync(0xffffffffu, wb_v);
     sb_v = __reduce_max_sync(0xffffffffu, sb_v);
@@ -303,7 +323,7 @@ __global__ void __launch_bounds__(PREP_THREADS) k_prep(Geo g, Ws w, long long pe
     __syncthreads();
     if (smem_hist) {
       for (int t = threadIdx.x; t < nd; t += blockDim.x)
-        if (s_diff[t]) atomicAdd(&w.tile_diff[G.diff0 + t], s_diff[t]);
+        if (s_diff[t]) atomicAdd(&w.tile_diff[w.gal[gk].diff0 + t], s_diff[t]);
       __syncthreads();
     }
     run0 = run_hi;
@@ -692,14 +712,19 @@ void launch_prep(const Geo& g, const Ws& w, int num_sms, cudaStream_t s, long lo
       k_table_finite<<<grid_for(g.n * 32, num_sms), 256, 0, s>>>(g, w);
     // every block adds its arrays to the global ones: fewer, longer runs where
     // the arrays are large
-    const int nd = g.max_diff <= PREP_SMEM_DIFF ? g.max_diff : g.ngal > 1 ? PREP_SMEM_DIFF : 0;
+    const bool runs = g.ngal == 1 || g.n > PREP_FEW * g.ngal;
+    const int nd = !runs                          ? 0
+                   : g.max_diff <= PREP_SMEM_DIFF ? g.max_diff
+                   : g.ngal > 1                   ? PREP_SMEM_DIFF
+                                                  : 0;
     const size_t hist_bytes = sizeof(int) * (size_t)nd;
     long long blocks = grid_for(g.n, num_sms);
     const long long most = (hist_bytes <= 16384 ? 8ll : 4ll) * num_sms;
     if (blocks > most) blocks = most;
     const long long per =
         ((g.n + blocks - 1) / blocks + PREP_THREADS - 1) / PREP_THREADS * PREP_THREADS;
-    k_prep<<<(unsigned)((g.n + per - 1) / per), PREP_THREADS, hist_bytes, s>>>(g, w, per);
+    (runs ? k_prep<true> : k_prep<false>)<<<(unsigned)((g.n + per - 1) / per), PREP_THREADS,
+                                            hist_bytes, s>>>(g, w, per);
   }
   launch_scan(w.npairs, g.n, w.pair_off, w.scan_sums, &w.hdr->n_pairs, s);
   // per-cube prefix sums of the difference arrays, in up to 200 KB of
