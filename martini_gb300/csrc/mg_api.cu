@@ -39,13 +39,13 @@ bool known_form(int form) {
 // Segment shape of a contraction form: channel blocks per tile and their
 // width.  Tensor-core forms: the band (rounded to 16) in one block up to 256
 // channels, else blocks of 256 (a block's master accumulator takes half of
-// the 512 TMEM columns).  `small_partials` (the built-in scratch of
-// mg_insert_noalloc) keeps the three-piece form at blocks of 128, whose
-// split-K partial tiles take half the room: a problem that fits the fixed
-// array with them may not fit with 256.
-void seg_shape(int form, int nc, bool small_partials, int* ncb, int* width) {
+// the 512 TMEM columns).  `narrow` keeps the three-piece form at blocks of 128:
+// for the built-in scratch of mg_insert_noalloc, because their split-K partial
+// tiles take half the room (a problem that fits the fixed array with them may
+// not fit with 256), and for tabulated spectra on few segments (NARROW_SEGS).
+void seg_shape(int form, int nc, bool narrow, int* ncb, int* width) {
   if (form == MG_FORM_BF16X3 || form == MG_FORM_F16X3 || form == MG_FORM_BF16X6) {
-    const int bw = small_partials && form == MG_FORM_BF16X6 ? 128 : 256;
+    const int bw = narrow && form == MG_FORM_BF16X6 ? 128 : 256;
     if (nc <= bw) {
       *ncb = 1;
       *width = (nc + 15) / 16 * 16;
@@ -57,6 +57,23 @@ void seg_shape(int form, int nc, bool small_partials, int* ncb, int* width) {
     *ncb = (nc + CBLK - 1) / CBLK;
     *width = CBLK;
   }
+}
+
+// A tabulated spectrum meets every channel block, so that blocks of 256 save no
+// work, and where a cube has few pixels their segments leave SMs idle: below half
+// of this part's 152 SMs the blocks are 128 wide.  Insertions (planned) with blocks
+// of 256 and 128: 10k particles on 27 x 10 x 508 (8 segments) 571 and 404 us, 20k
+// on 64 x 64 x 256 (32) 565 and 401, 150k on 64 x 64 x 512 (64) 1721 and 1653; 100k
+// on 128 x 64 x 512 (128) 1046 and 1060, 200k on 128 x 128 x 256 (128) 1089 and 1135.
+constexpr long long NARROW_SEGS = 76;
+
+// Whether a batch of tabulated spectra in the three-piece form falls under it.
+bool few_segments(const mg_problem* probs, int nprob) {
+  long long wide = 0;
+  for (int k = 0; k < nprob && wide < NARROW_SEGS; ++k)
+    wide += (long long)((probs[k].nx + TILE_I - 1) / TILE_I) *
+            ((probs[k].ny + TILE_J - 1) / TILE_J) * ((probs[k].nc + 255) / 256);
+  return wide < NARROW_SEGS;
 }
 
 int channel_bits(int nc) {
@@ -237,9 +254,10 @@ struct Batch {
 // Validate a batch (every cube shares the kernel table, spectral model,
 // contraction form and accumulate flag) and lay its cubes out in the
 // batch-wide index spaces.  `shape_only` (workspace sizing) checks just
-// what the layout depends on: sizes, pads and form.
+// what the layout depends on: sizes, pads and form.  `narrow`: blocks of 128
+// channels whatever the spectra (seg_shape).
 int make_batch(const mg_problem* probs, int nprob, Batch* b, bool shape_only = false,
-               bool small_partials = false) {
+               bool narrow = false) {
   if (!probs || nprob < 1) return fail(MG_ERR_INVALID_ARGUMENT, "empty batch");
   if (nprob > 65535) return fail(MG_ERR_INVALID_ARGUMENT, "at most 65535 cubes in a batch");
   for (int k = 0; k < nprob; ++k) {
@@ -282,6 +300,8 @@ int make_batch(const mg_problem* probs, int nprob, Batch* b, bool shape_only = f
     g.ks[k].truncate = p0.kernels[k].truncate;
     g.ks[k].gnorm = t == MG_KERNEL_GAUSSIAN ? (float)gaussian_norm(p0.kernels[k].truncate) : 1.f;
   }
+  if (!shape_only && p0.spectral_model == MG_SPECTRUM_TABLE && few_segments(probs, nprob))
+    narrow = true;
   b->gal.assign(nprob, Gal());
   long long n = 0, ndiff = 0, nedge = 0, nfpart = 0, ntiles = 0, nseg = 0, nrows = 0;
   for (int k = 0; k < nprob; ++k) {
@@ -309,7 +329,7 @@ int make_batch(const mg_problem* probs, int nprob, Batch* b, bool shape_only = f
     G.ntx = (p.nx + TILE_I - 1) / TILE_I;
     G.nty = (p.ny + TILE_J - 1) / TILE_J;
     const long long nt = (long long)G.ntx * G.nty;
-    seg_shape(p.form, p.nc, small_partials, &G.ncb, &G.width);
+    seg_shape(p.form, p.nc, narrow, &G.ncb, &G.width);
     G.p0 = n;
     G.n = p.n;
     G.tile0 = (int)ntiles;
@@ -409,6 +429,13 @@ int mg_workspace_size_batched(const mg_problem* probs, int32_t nprob, int64_t ma
   int rc = make_batch(probs, nprob, &b, true);
   if (rc) return rc;
   *bytes = layout(b.g, max_pairs, max_partial_items).total;
+  // a size serves every spectral model (the narrow blocks have more segments)
+  if (few_segments(probs, nprob)) {
+    Batch nb;
+    rc = make_batch(probs, nprob, &nb, true, true);
+    if (rc) return rc;
+    *bytes = std::max(*bytes, layout(nb.g, max_pairs, max_partial_items).total);
+  }
   return MG_OK;
 }
 
