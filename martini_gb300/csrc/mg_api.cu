@@ -42,7 +42,7 @@ bool known_form(int form) {
 // the 512 TMEM columns).  `narrow` keeps the three-piece form at blocks of 128:
 // for the built-in scratch of mg_insert_noalloc, because their split-K partial
 // tiles take half the room (a problem that fits the fixed array with them may
-// not fit with 256), and for tabulated spectra on few segments (NARROW_SEGS).
+// not fit with 256), and where narrow_blocks says so.
 void seg_shape(int form, int nc, bool narrow, int* ncb, int* width) {
   if (form == MG_FORM_BF16X3 || form == MG_FORM_F16X3 || form == MG_FORM_BF16X6) {
     const int bw = narrow && form == MG_FORM_BF16X6 ? 128 : 256;
@@ -59,21 +59,31 @@ void seg_shape(int form, int nc, bool narrow, int* ncb, int* width) {
   }
 }
 
-// A tabulated spectrum meets every channel block, so that blocks of 256 save no
-// work, and where a cube has few pixels their segments leave SMs idle: below half
-// of this part's 152 SMs the blocks are 128 wide.  Insertions (planned) with blocks
-// of 256 and 128: 10k particles on 27 x 10 x 508 (8 segments) 571 and 404 us, 20k
-// on 64 x 64 x 256 (32) 565 and 401, 150k on 64 x 64 x 512 (64) 1721 and 1653; 100k
-// on 128 x 64 x 512 (128) 1046 and 1060, 200k on 128 x 128 x 256 (128) 1089 and 1135.
-constexpr long long NARROW_SEGS = 76;
+// Blocks of 256 channels save the pairs of lines that straddle two of 128, but
+// halve the segments, and where there are few of those and too few pairs to split
+// them, SMs idle (and a line wider than 128 channels saves nothing).  Below two
+// segments for each of this part's 152 SMs the blocks are 128 wide, unless there
+// are particles enough (NARROW_N) to split.  Tabulated spectra save nothing on any
+// cube: below half a segment an SM they take blocks of 128 whatever the particles,
+// most of which may miss the cube.  Planned insertions with blocks of 256 and 128:
+// 35k wide lines on 103 x 130 x 318 (234 segments) 647 and 473 us (599 before there
+// were blocks of 256), 93k on 13 x 9 x 363 (4) 622 and 494 (552), 1.2M lines of 75
+// channels on 156 x 31 x 1039 (200) 2557 and 2770; tabulated, 20k on 64 x 64 x 256
+// (32) 565 and 401 us, 248k on 14 x 16 x 403 (4) 550 and 435.  Of 313 drawn calls under
+// the rule 9 are more than 3 % slower with blocks of 128 and the mean is 5 % faster;
+// 18 were slower than before there were blocks of 256, by up to 35 %, now 3, by up
+// to 4 %.
+constexpr long long NARROW_SEGS = 304, NARROW_SEGS_TABLE = 76;
+constexpr long long NARROW_N = 200000;
 
-// Whether a batch of tabulated spectra in the three-piece form falls under it.
-bool few_segments(const mg_problem* probs, int nprob) {
-  long long wide = 0;
-  for (int k = 0; k < nprob && wide < NARROW_SEGS; ++k)
+bool narrow_blocks(const mg_problem* probs, int nprob, bool table) {
+  long long wide = 0, n = 0;
+  for (int k = 0; k < nprob && wide < NARROW_SEGS; ++k) {
     wide += (long long)((probs[k].nx + TILE_I - 1) / TILE_I) *
             ((probs[k].ny + TILE_J - 1) / TILE_J) * ((probs[k].nc + 255) / 256);
-  return wide < NARROW_SEGS;
+    n += probs[k].n;
+  }
+  return wide < (n < NARROW_N ? NARROW_SEGS : table ? NARROW_SEGS_TABLE : 0);
 }
 
 int channel_bits(int nc) {
@@ -300,8 +310,8 @@ int make_batch(const mg_problem* probs, int nprob, Batch* b, bool shape_only = f
     g.ks[k].truncate = p0.kernels[k].truncate;
     g.ks[k].gnorm = t == MG_KERNEL_GAUSSIAN ? (float)gaussian_norm(p0.kernels[k].truncate) : 1.f;
   }
-  if (!shape_only && p0.spectral_model == MG_SPECTRUM_TABLE && few_segments(probs, nprob))
-    narrow = true;
+  narrow = narrow || narrow_blocks(probs, nprob,
+                                   !shape_only && p0.spectral_model == MG_SPECTRUM_TABLE);
   b->gal.assign(nprob, Gal());
   long long n = 0, ndiff = 0, nedge = 0, nfpart = 0, ntiles = 0, nseg = 0, nrows = 0;
   for (int k = 0; k < nprob; ++k) {
@@ -430,7 +440,7 @@ int mg_workspace_size_batched(const mg_problem* probs, int32_t nprob, int64_t ma
   if (rc) return rc;
   *bytes = layout(b.g, max_pairs, max_partial_items).total;
   // a size serves every spectral model (the narrow blocks have more segments)
-  if (few_segments(probs, nprob)) {
+  if (narrow_blocks(probs, nprob, true)) {
     Batch nb;
     rc = make_batch(probs, nprob, &nb, true, true);
     if (rc) return rc;
