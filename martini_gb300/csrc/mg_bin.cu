@@ -134,13 +134,12 @@ __device__ __forceinline__ bool certainly_off(double x, double r, int n) {
 
 // Whether a particle's tabulated spectrum holds a value that reach2 takes for
 // not finite, into the pair counts (which the records kernel reads and
-// overwrites); a warp per particle.  One more pass over the table, bound by
-// HBM: 57 us for 500k spectra of 128 channels (bf16x6 insertion 1.34 to 1.40
-// ms; 1.60 ms with the whole box of every particle listed).  Spectra of particles
-// a pixel or more off the cube, which have no pairs, are not read: 578k spectra of
-// 173 channels that nearly all miss it 374 to 276 us an insertion.
-// `group` particles a warp at a time: 8 share the latency of their positions, or 1
-// where there are warps enough for a particle each.
+// overwrites).  One more pass over the table, bound by HBM where it is long:
+// a warp takes `group` particles, whose rows are contiguous, and streams them
+// from the first to the last whose box may reach the cube (the others have no
+// pairs).  bf16x6 insertions without the pass and with it: 500k spectra of 128
+// channels on 200 x 200 962 and 1025 us, nearly all of them off the cube 264 and
+// 275; 2M of 16 channels on 300 x 300 1853 and 1908, with a warp per row 2016.
 __global__ void k_table_finite(Geo g, Ws w, int group) {
   const int lane = threadIdx.x & 31;
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
@@ -153,16 +152,33 @@ __global__ void k_table_finite(Geo g, Ws w, int group) {
       const long long p = P - G.p0;
       on = !certainly_off(G.x[p], G.r[p], G.nx) && !certainly_off(G.y[p], G.r[p], G.ny);
     }
-    unsigned bad_of = 0u;  // bit k: particle base + k
-    for (unsigned m = __ballot_sync(0xffffffffu, on); m; m &= m - 1) {
-      const int k = __ffs(m) - 1;
-      const Gal& G = w.gal[find_gal(w.gp0, g.ngal, base + k)];
-      const float* s = G.spectra + (base + k - G.p0) * G.nc;
-      bool bad = false;
-      for (int c = lane; c < G.nc; c += 32) bad |= !(fabsf(s[c]) < 1e30f);
-      if (__any_sync(0xffffffffu, bad)) bad_of |= 1u << k;
+    unsigned bad = 0u;  // bit k: particle base + k
+    for (unsigned m = __ballot_sync(0xffffffffu, on); m;) {
+      // rows k0 .. k1 - 1: those of the first wanted one's cube
+      const int k0 = __ffs(m) - 1;
+      const int gk = find_gal(w.gp0, g.ngal, base + k0);
+      const Gal& G = w.gal[gk];
+      const int k1 = (int)min((long long)(32 - __clz(m)), w.gp0[gk + 1] - base);
+      m = k1 < 32 ? m >> k1 << k1 : 0u;
+      const int nc = G.nc;
+      const float* const s = G.spectra + (base + k0 - G.p0) * nc;
+      const long long total = (long long)(k1 - k0) * nc;
+      for (long long e = lane; e < total; e += 256) {
+        float v[8];
+        bool any = false;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = e + 32 * j < total ? __ldg(s + e + 32 * j) : 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) any |= !(fabsf(v[j]) < 1e30f);
+        if (any) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (!(fabsf(v[j]) < 1e30f)) bad |= 1u << (k0 + (int)((e + 32 * j) / nc));
+        }
+      }
     }
-    if (lane < group && P < g.n) w.npairs[P] = (bad_of >> lane) & 1u;
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if (lane < group && P < g.n) w.npairs[P] = (bad >> lane) & 1u;
   }
 }
 
@@ -740,7 +756,8 @@ void launch_prep(const Geo& g, const Ws& w, int num_sms, cudaStream_t s, long lo
   k_edges<<<grid_for(g.nedge, num_sms), 256, 0, s>>>(g, w);
   if (g.n > 0) {
     if (g.spectral_model == MG_SPECTRUM_TABLE) {
-      const int group = g.n > (long long)num_sms * 512 ? 8 : 1;
+      // 32 particles a warp, fewer while that leaves SMs with few warps
+      const int group = (int)std::min<long long>(32, 1 + g.n / (num_sms * 32ll));
       k_table_finite<<<grid_for((g.n + group - 1) / group * 32, num_sms), 256, 0, s>>>(g, w, group);
     }
     // every block adds its arrays to the global ones: fewer, longer runs where

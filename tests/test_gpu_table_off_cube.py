@@ -75,3 +75,39 @@ def test_spectra_off_the_cube_cost_little():
             t.append(a.elapsed_time(b) * 1e3)
         us.append(sorted(t)[7])
     assert us[1] <= us[0] + 50.0, us  # 800 MB against 8
+
+
+@pytest.mark.parametrize("n,nc", [(5, 1), (31, 3), (33, 33), (4900, 2), (20000, 7), (165000, 3),
+                                  (300000, 1)])
+@pytest.mark.parametrize("cubes", [1, 3])
+def test_the_value_is_found_in_its_row(n, nc, cubes):
+    import torch
+    from martini_gb300 import _native as N
+    from martini_gb300.engine import DeviceParticles, InsertionEngine, insert_batch
+    eng = InsertionEngine("cuda:0")
+    rng = np.random.default_rng(n + nc)
+    items, boxes = [], []
+    for k in range(cubes):  # cubes of n, n + 7, n + 14 particles
+        m = n + 7 * k
+        x, y = rng.uniform(100, 900, m), rng.uniform(0, NY - 1, m)  # off the cube but for four
+        h = np.ones(m)
+        rows = np.unique(np.concatenate([[0, m - 1], rng.integers(0, m, 2)]))
+        x[rows] = [5.0, 17.0, 30.0, 42.0][:rows.size]
+        y[rows], h[rows] = 20.0, 1.5
+        table = rng.random((m, nc)).astype(np.float32)
+        bad = rows[k % rows.size]
+        table[bad, k % nc] = np.inf
+        parts = DeviceParticles.from_host(eng.device, x, y, np.full(m, 3.0), h, None, spectra=table)
+        edges = torch.from_numpy(np.arange(nc + 1) * 4.0).to(eng.device)
+        items.append(dict(parts=parts, edges=edges, nx=NX, ny=NY, nc=nc))
+        i, j = np.arange(NX)[:, None], np.arange(NY)[None, :]
+        boxes.append(((np.abs(i - x[bad]) <= 3) & (np.abs(j - 20.0) <= 3), k % nc))
+    outs = insert_batch(eng, items, [(N.MG_KERNEL_CUBIC_SPLINE, 0.0)], N.MG_SPECTRUM_TABLE,
+                        form=N.MG_FORM_FP32)
+    for (cube, _), (box, c) in zip(outs, boxes):
+        got = cube.cpu().numpy()
+        assert np.isnan(got[..., c][box]).any() and not np.isfinite(got[..., c][box]).any()
+        tiles = np.zeros((NX, NY), bool)  # tiles of 8 x 16 pixels that meet the box
+        for i, j in zip(*np.nonzero(box)):
+            tiles[i // 8 * 8:i // 8 * 8 + 8, j // 16 * 16:j // 16 * 16 + 16] = True
+        assert np.isfinite(got[~tiles]).all()
