@@ -1337,8 +1337,9 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
   unsigned full_par = 0u, parb_par = 0u;
   int stage = 0;
   int since_drain = 0;
-  // thread 0 takes the next item from the queue while this one runs (the
-  // atomic's round trip is off the item switch)
+  // Thread 0 takes the next item from the queue at the end of this one's stages.
+  // Taken at its start, the CTAs that start first hold two items each where there
+  // are few, and others none or, a round later, a third.
   long long next_item = tid == 0 ? (long long)atomicAdd(&w.hdr->item_counter, 1u) : 0;
 
   for (;;) {
@@ -1346,7 +1347,6 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
     __syncthreads();
     const long long item = s_item;
     if (item >= n_items || s_abort) break;
-    if (tid == 0) next_item = (long long)atomicAdd(&w.hdr->item_counter, 1u);
     // the queue runs over the items in cost order, largest first
     const ItemTC it = decode_tc(g, w, (long long)w.item_order[item], kch);
     const Gal& G = w.gal[it.gal];
@@ -1629,6 +1629,8 @@ k_contract_tc(Geo g, Ws w, int nwmax) {
       }
     }
     since_drain = 0;
+    // the next item: the round trip passes behind the last MMAs and the epilogue
+    if (tid == 0) next_item = (long long)atomicAdd(&w.hdr->item_counter, 1u);
 
     // all MMAs of the item complete (a commit covers every earlier MMA)
     for (int s = 0; s < 2; ++s) {
