@@ -116,7 +116,8 @@ typedef struct mg_plan_info {
   int64_t n_partial_items;  /* upper bound on split-K partial tiles */
   int64_t n_tiles;
   size_t workspace_bytes;   /* mg_workspace_size(p, n_pairs, n_partial_items), plus the
-                               spectrum store of the tensor-core forms (not TABLE) */
+                               spectrum store (GAUSSIAN and DIRAC models, every form): 4
+                               bytes for each channel of each particle's line */
 } mg_plan_info;
 
 /* Library version string. */
@@ -151,10 +152,11 @@ int mg_plan(const mg_problem* p, void* workspace, size_t workspace_bytes, void* 
  * the same max_pairs / max_partial_items.  If the data need more than that,
  * the device code skips the contraction and mg_check() returns
  * MG_ERR_WORKSPACE.  Bytes beyond mg_workspace_size(p, max_pairs,
- * max_partial_items) hold the per-particle spectrum store of the tensor-core
- * forms (Gaussian and Dirac lines, computed once per particle, not once per
- * tile); mg_plan's workspace_bytes has room for it.  With less room the
- * lines are evaluated inside the contraction: same results, slower.
+ * max_partial_items) hold the per-particle spectrum store (Gaussian and Dirac
+ * lines of every form, computed once per particle, not once per tile); mg_plan's
+ * workspace_bytes has room for it.  With less room (mg_workspace_size's bytes,
+ * say, where the store of many wide lines cannot be allocated) the lines are
+ * evaluated inside the contraction: same results, slower.
  */
 int mg_insert(const mg_problem* p, void* workspace, size_t workspace_bytes, int64_t max_pairs,
               int64_t max_partial_items, void* stream);
@@ -163,7 +165,7 @@ int mg_insert(const mg_problem* p, void* workspace, size_t workspace_bytes, int6
 #define MG_STAGE_BIN 1        /* records, tile histogram, plan, tile-major list */
 #define MG_STAGE_CONTRACT 2   /* cube clear, contraction, split-K reduction */
 #define MG_STAGE_FLUX 4       /* FP64 flux sums (if p->flux) */
-#define MG_STAGE_SPEC 8       /* per-particle spectrum store (tensor-core forms, not TABLE
+#define MG_STAGE_SPEC 8       /* per-particle spectrum store (GAUSSIAN and DIRAC
                                  models; runs between BIN and CONTRACT; a BIN stage
                                  invalidates it, and CONTRACT then evaluates in-kernel) */
 #define MG_STAGE_ALL 15

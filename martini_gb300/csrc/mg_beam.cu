@@ -16,8 +16,8 @@
 // memory once for many of them: a lane loads a window of 16 + T - 1 pixels and
 // applies T = 8 taps of two kernel rows to it, 128 paired FMAs for 23 loads (one
 // load per FMA before: 9.70 ms on 512 x 512 x 256 with a 27 px beam; now
-// 2.16 ms, 1.23 ms of it at the FP32 FMA rate).  Input rows stream through a ring in shared memory (cp.async,
-// BR_AHEAD rows ahead): at step s warp w takes input row 2 w + s, so that every
+// 2.21 ms, 1.23 ms of it at the FP32 FMA rate).  Input rows stream through a ring
+// in shared memory (cp.async, BR_AHEAD rows ahead): at step s warp w takes input row 2 w + s, so that every
 // warp works on kernel rows kx - 1 - s and kx - s and only 15 rows are live.
 // That leaves room for two blocks on an SM, and the ring's size depends on ky
 // mostly, so beams up to 71 px take this path whole (27 px before).  Wider ones

@@ -67,11 +67,12 @@ void launch_set_gals(const Gal* gals, const Geo& g, const Ws& w, cudaStream_t s)
 // fits (PREP_SMEM_DIFF) lives in shared memory meanwhile and is added to the
 // global one once per block and cube, and the cube's maxima are reduced in
 // registers first.  (Small cubes have few counters, and 7 million particles of
-// a 48-galaxy batch met on them in global memory: 1.77 ms, 0.81 ms then.)
-// What bounds it is the FP64 pipe (83 % busy with about 70 instructions a
-// particle): the comparisons of FP64 values are made on their bits instead, and
-// starting points and guesses come from FP32 (4M particles in 1024^2 x 512:
-// 0.58 ms, 0.34 ms now; 1M particles 0.14 and 0.09 ms).
+// a 48-galaxy batch met on them in global memory: 1.77 ms with all counters there,
+// 0.81 ms with the arrays in shared memory.)  The FP64 pipe bounds it (83 % busy
+// with about 70 instructions a particle), so the comparisons of FP64 values are
+// made on their bits and starting points and guesses come from FP32: 4M particles
+// in 1024^2 x 512 0.58 ms before and 0.34 ms with both, 1M particles 0.14 and 0.09,
+// the batch 0.81 and 0.44.
 
 // The tiles a particle is listed for: those of its footprint box that hold a
 // pixel within the kernel's support radius, so the tiles in the corners of a
@@ -509,7 +510,8 @@ __global__ void k_plan_finish(Geo g, Ws w, int num_sms, unsigned long long plan_
 // stand, the header takes the capacities and the launch shape of this run.
 // The later stages overwrite the counts, so a plan serves one run.  A binning
 // pass less in a call that plans first: 1M particles 6.01 to 5.80 ms, 5k particles
-// 0.42 to 0.38 ms.
+// 0.42 to 0.38 ms.  For an engine's later calls only: where the workspace grows
+// after the plan, as in the first call, the run bins again.
 __global__ void k_resume(Geo g, Ws w, int num_sms, long long cap_pairs, long long cap_partial,
                          unsigned long long plan_key) {
   WsHeader* h = w.hdr;
@@ -798,6 +800,9 @@ int seg_bits(const Geo& g) {
   return b;
 }
 
+// Bits of a key of segment, kernel class and first channel.  Problems past 32 are
+// refused: the list's keys held all three once.  They hold the segment alone now;
+// the limit stands as part of the interface.
 int sort_bits(const Geo& g) { return seg_bits(g) + g.cbits; }
 
 // The list sorted by segment, then class and first channel, then the segments

@@ -6,13 +6,14 @@
 // output tiles: a pixel's spectrum is the sum over the particles whose
 // footprint box contains it of weight * spectrum.
 //
-// Bound by issue slots and the latency between barriers.  A chunk's records
+// Bound by latency: 51 % of issue slots used with three blocks on an SM, warps
+// waiting for shared memory and the table's cells most.  A chunk's records
 // and spectrum-store rows are copied while the chunk before is multiplied, the
 // lines come from the store (once per particle instead of once per tile), the
 // weights are taken by whole warps with what a particle's pixels share computed
 // once, and the FMAs work on pairs of pixels; three blocks fit on an SM.  100k
-// quartic-spline particles in 256^2 x 128 (1.43M pairs): 2.09 ms before (1058
-// warp instructions a pair, of which 256 multiply), 1.10 ms now.
+// quartic-spline particles on 187 x 211 x 75 (1.44M pairs): 2.09 ms before (1058
+// warp instructions a pair, of which 256 multiply), 1.12 ms now (464).
 #include "mg_internal.cuh"
 
 namespace mg {

@@ -4,8 +4,10 @@
 // Bound by host memory (20 bytes a voxel: the array read and written, the
 // cube read) and by the FP64 divisions.  As whole-array operations (convert,
 // add, divide, multiply, sum twice) the same work made six passes and three
-// temporaries: the call on a 128^3 cube and 100k particles took 9.5 ms, of which
-// the GPU 0.9; 4.1 ms now (with the particle amplitudes' power as a division).
+// temporaries.  A call on a 128^3 cube and 100k particles (0.9 ms of it on the GPU),
+// with the particle amplitudes' power as a division too: the first of a new object
+// 10.6 ms before and 4.7 ms now, in a new process 19 and 6.3, repeated on one
+// object 9.0 and 4.4.
 // Pixel rows go to a few threads; each row's per-channel sums are kept apart
 // and added in row order, so the result does not depend on the thread count.
 #include <sys/mman.h>

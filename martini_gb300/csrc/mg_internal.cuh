@@ -37,7 +37,7 @@ __host__ __device__ inline int item_particles(long long total_pairs, int num_sms
   return (int)t;
 }
 
-// Per-particle record written by the prep kernel (64 bytes).
+// Per-particle record written by the prep kernel (72 bytes).
 struct __align__(8) PRec {
   int ilo, ihi, jlo, jhi;  // exact footprint box (inclusive), clipped; empty if ilo > ihi
   int xi, yi;              // floor(x), floor(y)
@@ -53,9 +53,9 @@ struct __align__(8) PRec {
 };
 
 // The footprint's rows [ilo, ihi] hold every cube row within the kernel's
-// support radius h of the particle (tested in FP64 with a 2^-20 margin, so
-// the FP32 profile argument of any other row is past the support): a radial
-// table kernel needs no per-row box test.
+// support radius h of the particle (tested in FP32 with a margin of 2^-18 and of
+// 1e-6 of the coordinate, so the FP32 profile argument of any other row is past
+// the support): a radial table kernel needs no per-row box test.
 constexpr int PREC_ROWS_COVER = 1;
 // The same for the footprint's columns [jlo, jhi] (axis 1).
 constexpr int PREC_COLS_COVER = 2;
@@ -143,7 +143,7 @@ struct Geo {
   int nseg;           // segments of all cubes
   int max_width;      // widest channel block (partial slots hold TILE_PX x max_width)
   int max_nc;
-  int cbits;          // class and channel bits of the order within a segment
+  int cbits;          // class and channel bits, for the size limit (sort_bits)
   int nrows;          // flux rows of all cubes
   int max_diff;       // largest difference array of one cube
   long long n;        // particles of all cubes
@@ -192,7 +192,7 @@ struct WsHeader {
   long long partial_bound;       // upper bound on partial items (from tile counts)
   long long cap_pairs;
   long long cap_partial_items;
-  long long spec_bound;          // sum over particles of support channels (Gaussian)
+  long long spec_bound;          // sum over particles of support channels (stored_lines)
   long long n_spec;              // values in the spectrum store (spectrum stage)
   int spec_ready;                // 1 once the store holds this binning's spectra
   int kch;                       // particles per work item (item_particles)
@@ -205,7 +205,7 @@ static_assert(sizeof(WsHeader) <= 256, "header slot of the workspace");
 // over the whole batch.  A "segment" is one (tile, channel block) of the
 // contraction: Gal::ncb blocks per tile (FP32 form: ceil(nc / CBLK) blocks
 // of CBLK channels; tensor-core forms: the band rounded to 16 in one block up
-// to 256 channels, else blocks of 256).
+// to 256 channels, else blocks of 256; 128 for both where seg_shape says so).
 struct Ws {
   WsHeader* hdr;
   Gal* gal;              // [ngal]
@@ -240,8 +240,8 @@ struct Ws {
   long long* part_off;   // [nseg] exclusive scan of seg_part
   float* partial;        // [cap_partial_items][TILE_PX][max_width]
   double* flux_part;     // [nfpart]
-  unsigned* spec;        // [cap_spec] per-particle Gaussian spectra over [clo, chi], as the
-                         // tensor-core form's scaled 16-bit hi | lo << 16 halves
+  unsigned* spec;        // [cap_spec] per-particle lines over [clo, chi]: FP32 values, or the
+                         // two-piece forms' scaled 16-bit hi | lo << 16 halves
   long long cap_spec;    // room in spec (the workspace beyond the fixed layout)
   // Work queue order: item_order[k] is the k-th item the contraction takes,
   // the items sorted by estimated cost, largest first (stable: equal costs
