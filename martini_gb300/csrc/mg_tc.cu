@@ -634,8 +634,14 @@ __global__ void k_spec_eval(Geo g, Ws w) {
 // Long lines are bound by the error functions, whose branches a warp's lanes
 // share best on one line: with one past 32 channels, the four in turn.
 // `quad`: 4, or 1 where there are warps enough for a particle each.
+// Not where particles have fewer than 1.75 pairs on average: most lines would be
+// read once, and the contraction evaluates them in less time (Dirac kernels, 847k
+// lines of 27 channels on 41 x 21 x 59, one pair each: insertion 1203 us with the
+// store, 1001 without; 300k with 1.4 pairs on 200 x 200 x 59 828 and 812, with 2.1
+// 1038 and 1076, of 136 channels 1071 and 1200).
 __global__ void k_spec_fp32(Geo g, Ws w, int quad) {
-  const bool fits = w.hdr->n_spec <= w.cap_spec && !(w.hdr->status & ST_NO_PLAN);
+  const bool fits = w.hdr->n_spec <= w.cap_spec && !(w.hdr->status & ST_NO_PLAN) &&
+                    4 * w.hdr->n_pairs >= 7 * w.hdr->n_valid;
   if (blockIdx.x == 0 && threadIdx.x == 0) w.hdr->spec_ready = fits ? 1 : 0;
   if (!fits) return;
   const int lane = threadIdx.x & 31;
