@@ -1,6 +1,7 @@
 // C ABI of the martini_gb300 library (declared in include/martini_gb300.h).
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -559,7 +560,8 @@ int run(const mg_problem* probs, int nprob, void* ws, size_t bytes, cudaStream_t
       }
     }
     if (e == cudaSuccess)
-      e = cudaMemsetAsync(&w.hdr->item_counter, 0, sizeof(unsigned) + sizeof(w.hdr->sm_blocks), s);
+      e = cudaMemsetAsync(&w.hdr->item_counter, 0,
+                          offsetof(WsHeader, n_pairs) - offsetof(WsHeader, item_counter), s);
     if (e != cudaSuccess) return cuda_fail(e, "cube clear");
     if (tc_form(g.form)) {
       rc = launch_contract_bf16x3(g, w, num_sms(), s);

@@ -87,6 +87,7 @@ k_contract_fp32(Geo g, Ws w) {
   __shared__ KSpec s_ks[MG_MAX_KERNELS];
   __shared__ long long s_item;
   __shared__ unsigned s_rank;
+  __shared__ int s_next;  // where this block takes its items from (take)
 
   const int tid = threadIdx.x;
   if (tid < MG_MAX_KERNELS) s_ks[tid] = g.ks[tid];
@@ -107,7 +108,40 @@ k_contract_fp32(Geo g, Ws w) {
     s_rank = (atomicAdd(&w.hdr->sm_blocks[id >> 2], 1u << sh) >> sh) & 255u;
   }
   __syncthreads();
-  if ((long long)s_rank * (gridDim.x / F32_BLOCKS_PER_SM) >= n_items) return;
+  const int nsm = gridDim.x / F32_BLOCKS_PER_SM;
+  if ((long long)s_rank * nsm >= n_items) return;
+  // The queue's items in cost order, largest first.  The first nsm of them go to
+  // the blocks that are the first of their SM, the next nsm to the second blocks
+  // (smallest first) and so on, so that an SM does not start on three large ones
+  // while another has three small; then whichever block is free takes the next, and
+  // in the end what is left of the first ones.  305k particles with Dirac lines on
+  // 98 x 9 x 2406 (items of 1 to 2048 particles): contraction 835 us with one
+  // cursor, 700 now.
+  auto first_item = [&](int r) -> long long {  // of the blocks that are the r-th of their SM
+    const long long m = min((long long)nsm, n_items - (long long)r * nsm);
+    const int sh = 21 * r;
+    const long long c = (atomicAdd(&w.hdr->first_items, 1ull << sh) >> sh) & 0x1fffffull;
+    return c < m ? (long long)r * nsm + (r == 1 ? m - 1 - c : c) : -1;
+  };
+  auto take = [&]() -> long long {  // by one thread; n_items: none left
+    if (s_next < 0) {
+      s_next = 0;
+      const long long f = s_rank < F32_BLOCKS_PER_SM ? first_item((int)s_rank) : -1;
+      if (f >= 0) return f;
+    }
+    if (s_next == 0) {
+      const long long q = (long long)F32_BLOCKS_PER_SM * nsm +
+                          (long long)atomicAdd(&w.hdr->item_counter, 1u);
+      if (q < n_items) return q;
+      s_next = 1;
+    }
+    for (; s_next <= F32_BLOCKS_PER_SM; ++s_next) {
+      const long long f = first_item(s_next - 1);
+      if (f >= 0) return f;
+    }
+    return n_items;
+  };
+  if (tid == 0) s_next = -1;
   const int kch = hdr->kch;
   const unsigned* spec = stored_lines(g.spectral_model) && w.cap_spec > 0 && hdr->spec_ready
                              ? w.spec
@@ -117,7 +151,7 @@ k_contract_fp32(Geo g, Ws w) {
   const int tc = tid & 15;  // channel group: channels tc*4 .. tc*4+3
 
   for (;;) {
-    if (tid == 0) s_item = (long long)atomicAdd(&w.hdr->item_counter, 1u);
+    if (tid == 0) s_item = take();
     __syncthreads();
     const long long item = s_item;
     __syncthreads();

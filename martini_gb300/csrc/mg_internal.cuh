@@ -186,6 +186,8 @@ struct WsHeader {
   unsigned int item_counter;     // dynamic scheduler cursor
   unsigned int sm_blocks[SM_BUCKETS / 4];  // blocks of the FP32 contraction started on each
                                            // SM, a byte each; cleared with the cursor
+  unsigned long long first_items;  // its first items taken: 21 bits for each of the three
+                                   // blocks of an SM; cleared with the cursor
   long long n_pairs;
   long long n_items;
   long long n_partial_items;
