@@ -638,10 +638,12 @@ __global__ void k_spec_eval(Geo g, Ws w) {
 // read once, and the contraction evaluates them in less time (Dirac kernels, 847k
 // lines of 27 channels on 41 x 21 x 59, one pair each: insertion 1203 us with the
 // store, 1001 without; 300k with 1.4 pairs on 200 x 200 x 59 828 and 812, with 2.1
-// 1038 and 1076, of 136 channels 1071 and 1200).
+// 1038 and 1076, of 136 channels 1071 and 1200).  With fewer items than SMs the
+// store is filled by the whole chip and the contraction by a part: 20k with 1.6 pairs
+// on 60 x 60 x 64 676 us with the store, 700 without.
 __global__ void k_spec_fp32(Geo g, Ws w, int quad) {
   const bool fits = w.hdr->n_spec <= w.cap_spec && !(w.hdr->status & ST_NO_PLAN) &&
-                    4 * w.hdr->n_pairs >= 7 * w.hdr->n_valid;
+                    (4 * w.hdr->n_pairs >= 7 * w.hdr->n_valid || w.hdr->n_items < SM_BUCKETS);
   if (blockIdx.x == 0 && threadIdx.x == 0) w.hdr->spec_ready = fits ? 1 : 0;
   if (!fits) return;
   const int lane = threadIdx.x & 31;

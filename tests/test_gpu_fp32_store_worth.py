@@ -1,9 +1,10 @@
 """The FP32 form evaluates Gaussian lines in the contraction where particles meet
 few tiles and keeps them per particle where they meet more: the same bits either
 way, on both sides of 1.75 pairs a particle, and particles with one tile pay for
-no store."""
+no store, unless there are fewer work items than SMs."""
 
-import numpy as np
+import ctypes as C
+
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -63,3 +64,27 @@ def test_one_tile_each_pays_for_no_store():
             t.append(a.elapsed_time(b) * 1e3)
         us.append(sorted(t)[5])
     assert us[0] <= us[1] + 90.0, us  # 240 us more with the store
+
+
+@pytest.mark.parametrize("nx,ny,stored", [(60, 60, True), (200, 200, False)])
+def test_few_items_keep_the_store(nx, ny, stored):
+    import torch
+    from martini_gb300 import _native as N
+    from martini_gb300.engine import InsertionEngine
+    eng = InsertionEngine("cuda:0")
+    prob, cube, ratio, keep = planned(eng, 40000 if stored else 30000, nx, ny, 64, 1.0,
+                                      N.MG_KERNEL_CUBIC_SPLINE, 12.0)
+    assert ratio <= 1.75
+    eng.run(prob)
+    eng.check()
+    want = cube.clone()
+    used = eng.last_plan.workspace_bytes
+    size = C.c_size_t()
+    N.check(eng.lib.mg_workspace_size(C.byref(prob), *eng._caps,
+                                      C.byref(size)))
+    assert used > size.value  # the plan has room for the store either way
+    eng._ws[size.value:used] = 255
+    eng.run(prob)
+    eng.check()
+    assert torch.equal(cube, want)
+    assert bool((eng._ws[size.value:used] != 255).any()) == stored
