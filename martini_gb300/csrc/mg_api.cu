@@ -61,21 +61,19 @@ void seg_shape(int form, int nc, bool narrow, int* ncb, int* width) {
 }
 
 // Blocks of 256 channels save the pairs of lines that straddle two of 128, but
-// halve the segments, and where there are few of those and too few pairs to split
-// them, SMs idle (and a line wider than 128 channels saves nothing).  Below two
-// segments for each of this part's 152 SMs the blocks are 128 wide, unless there
-// are particles enough (NARROW_N) to split.  Tabulated spectra save nothing on any
-// cube: below half a segment an SM they take blocks of 128 whatever the particles,
-// most of which may miss the cube.  Planned insertions with blocks of 256 and 128:
-// 35k wide lines on 103 x 130 x 318 (234 segments) 647 and 473 us (599 before there
-// were blocks of 256), 93k on 13 x 9 x 363 (4) 622 and 494 (552), 1.2M lines of 75
-// channels on 156 x 31 x 1039 (200) 2557 and 2770; tabulated, 20k on 64 x 64 x 256
-// (32) 565 and 401 us, 248k on 14 x 16 x 403 (4) 550 and 435.  Of 313 drawn calls under
-// the rule 9 are more than 3 % slower with blocks of 128 and the mean is 5 % faster;
-// 18 were slower than before there were blocks of 256, by up to 35 %, now 3, by up
-// to 4 %.
-constexpr long long NARROW_SEGS = 304, NARROW_SEGS_TABLE = 76;
-constexpr long long NARROW_N = 200000;
+// halve the segments; with few pairs a segment is one work item, and few segments
+// leave SMs idle.  Below two segments for each of this part's 152 SMs the blocks are
+// 128 wide, unless there are so many particles (NARROW_PER, an item's worth of pairs
+// in each) that segments are split anyway.  Tabulated spectra meet every block and
+// save nothing on any cube: below half a segment an SM they take blocks of 128
+// whatever the particles, most of which may miss the cube.  Insertions with blocks
+// of 256 and 128: lines, 20k particles on 57 x 70 x 187 (40 segments) 624 and 531 us,
+// 25k on 116 x 122 x 277 (240) 578 and 513; not taken: 80k on 87 x 56 x 213 (44)
+// 517 and 608, 169k on 95 x 70 x 292 (120) 1184 and 1417; tabulated, 20k on
+// 64 x 64 x 256 (32) 565 and 401, 248k on 14 x 16 x 403 (4) 550 and 435.  Lines wider
+// than 128 channels would gain with many particles too (93k on 13 x 9 x 363 622 and 494
+// us), but their widths are not known here.
+constexpr long long NARROW_SEGS = 304, NARROW_SEGS_TABLE = 76, NARROW_PER = 500;
 
 bool narrow_blocks(const mg_problem* probs, int nprob, bool table) {
   long long wide = 0, n = 0;
@@ -84,7 +82,7 @@ bool narrow_blocks(const mg_problem* probs, int nprob, bool table) {
             ((probs[k].ny + TILE_J - 1) / TILE_J) * ((probs[k].nc + 255) / 256);
     n += probs[k].n;
   }
-  return wide < (n < NARROW_N ? NARROW_SEGS : table ? NARROW_SEGS_TABLE : 0);
+  return wide < (n < NARROW_PER * wide ? NARROW_SEGS : table ? NARROW_SEGS_TABLE : 0);
 }
 
 int channel_bits(int nc) {
